@@ -25,6 +25,7 @@
 #include <algorithm>
 #include "ymkh_common.cuh"
 
+#include <cuda.h>
 #include <nvtx3/nvToolsExt.h>
 
 
@@ -91,6 +92,9 @@ struct ymkh_ctx {
   unsigned* derr = nullptr; // device error word of the bounded in-kernel waits
   RunDesc* ddesc = nullptr; // device run descriptors for start buffer 0 and 1
   RunDesc hdesc[2]{};       // their host copy, uploaded in stream order by the next step call
+  TensorMap* dmaps = nullptr; // device tensor maps: kFctMaps of buffer 0, then of buffer 1
+  TensorMap hmaps[2 * kFctMaps]{};  // their host copy, uploaded with hdesc
+  bool boxed = false;         // hmaps encoded: evenly spaced, 16-byte aligned arrays, nx even
   int fct_items = 0, mx_items = 0, fx_items = 0, fz_items = 0;
   bool desc_ok = false;
   bool desc_pending = false; // hdesc not yet uploaded to ddesc
@@ -231,17 +235,22 @@ int pick_segment(int nz, int nstrips, int grid) {
 }
 
 // One-row segments: a CTA's contiguous block then ends at any row, so the
-// blocks differ by at most one row (at 1024 x 2048 on B200 the step took
-// 0.523 ms against 0.529 ms with 16-row segments, 7.38 against 7.40 ms at
-// 4096 x 8192).  Maxwell keeps round-robin segments: its contiguous form
-// measured slower (7.49 ms).
+// blocks differ by at most one row.
 constexpr int kFctSegment = 1;
 
 void choose_launch_shape(ymkh_ctx* c) {
   cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->device);
-  // 128-wide strips from NX = 1024 up: at 4096 x 8192 on B200 the step's FCT
-  // + Maxwell take 6.97 + 2.80 ms against 7.31 + 3.09 ms with 64-wide strips
-  c->fct_tx = c->nx >= 1024 ? 128 : (c->nx >= 128 ? 64 : 32);
+  // Strip width.  Where rows come by TMA (periodic x, NX even) the 128-wide
+  // form is the faster one from NX = 128 up (FCT us, NZ x NX, 128- against
+  // 64-wide strips: 64 x 128 23 / 29, 256 x 512 47 / 48, 256 x 768 56 / 73,
+  // 2048 x 128 85 / 96) and below that from NZ = 256 up (512 x 64 35 / 44,
+  // but 64 x 96 28 / 24, where its row start-up shows).  Its element-wise
+  // copies (walls, odd NX) are issued by four of its sixteen warps: there it
+  // takes wide grids to win (walls, 256 x 513 77 / 63, 64 x 769 47 / 51,
+  // 512 x 1025 140 / 157).
+  const bool tma = c->sp.periodic_x && c->nx % 2 == 0;
+  const bool wide = tma ? (c->nx >= 128 || c->nz >= 256) : c->nx >= 768;
+  c->fct_tx = wide ? 128 : (c->nx >= 128 ? 64 : 32);
   const int fct_per_sm = std::max(1, fct_ctas_per_sm(c->fct_tx));
   c->fct_grid = c->sms * fct_per_sm;
   // segments are the FCT's unit of load balance: each CTA runs a contiguous
@@ -268,6 +277,10 @@ RunDesc make_desc(const ymkh_ctx* c, int start, int tb, int fct_item0, int mx_it
   d.fct_seg = c->fct_seg;
   d.fct_item0 = fct_item0;
   d.fct_bulk = (c->aligned16 && fct_bulk_ok(c->sp, tb)) ? kAlignedRowLoad : (int)LOAD_ELEM;
+  if (tb == 128 && d.fct_bulk != LOAD_ELEM && c->boxed) {
+    d.fct_bulk = LOAD_BOX;
+    d.maps = c->dmaps + kFctMaps * start;
+  }
   d.mx_nstrips = maxwell_nstrips(c->nx);
   d.mx_seg = c->mx_seg;
   d.mx_item0 = mx_item0;
@@ -297,12 +310,48 @@ int ensure_xscratch(ymkh_ctx* c) {
 int items_fct(const RunDesc& d, int nz) { return d.fct_nstrips * ((nz + d.fct_seg - 1) / d.fct_seg); }
 int items_mx(const RunDesc& d, int nz) { return d.mx_nstrips * ((nz + d.mx_seg - 1) / d.mx_seg); }
 
+// Tensor maps of both buffers for the FCT's TMA boxes: [array][z][x] with the
+// distance between arrays as the outer stride, which needs the 24 arrays of a
+// buffer evenly spaced in the state's order (a [24, NZ, NX] tensor, or the
+// library's own buffer).  Other layouts, odd NX and unaligned arrays keep the
+// per-array row copies.
+bool encode_box(TensorMap* out, const State& s, int nx, int nz, int arrays, int width) {
+  const double* p[24];
+  for (int i = 0; i < 12; ++i) p[i] = s.f[i];
+  for (int i = 0; i < 6; ++i) { p[12 + i] = s.a[i]; p[18 + i] = s.b[i]; }
+  const ptrdiff_t d = p[1] - p[0];
+  if (d < (ptrdiff_t)nx * nz) return false;
+  for (int i = 2; i < 24; ++i) if (p[i] - p[i - 1] != d) return false;
+  const cuuint64_t dims[3] = {(cuuint64_t)nx, (cuuint64_t)nz, 24};
+  const cuuint64_t strides[2] = {(cuuint64_t)nx * sizeof(double), (cuuint64_t)d * sizeof(double)};
+  if (strides[0] % 16 || strides[1] % 16 || strides[1] >= (1ull << 40)) return false;
+  const cuuint32_t box[3] = {(cuuint32_t)width, 1, (cuuint32_t)arrays}, es[3] = {1, 1, 1};
+  static const auto encode = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      fn = nullptr;
+    return reinterpret_cast<decltype(&cuTensorMapEncodeTiled)>(fn);
+  }();
+  static_assert(sizeof(CUtensorMap) == sizeof(TensorMap) && alignof(CUtensorMap) <= alignof(TensorMap), "tensor map");
+  if (!encode) return false;
+  return encode(reinterpret_cast<CUtensorMap*>(out), CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, const_cast<double*>(p[0]), dims,
+                strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // Device descriptors of this run for both start buffers (single-run tables).
 int upload_desc(ymkh_ctx* c) {
   c->desc_ok = false;
   if (!c->bound) return 0;
   if (!c->ddesc) CK(cudaMalloc(&c->ddesc, 2 * sizeof(RunDesc)), "cudaMalloc run descriptors");
   { int rc = ensure_xscratch(c); if (rc) return rc; }
+  c->boxed = c->aligned16 && c->nx >= kFctBoxWidth;
+  constexpr int arrays[kFctMaps] = {12, 9, 1, 12, 9}, width[kFctMaps] = {kFctBoxWidth, kFctBoxWidth, kFctBoxWidth, 4, 4};
+  for (int k = 0; k < 2 * kFctMaps && c->boxed; ++k)
+    c->boxed = encode_box(&c->hmaps[k], c->buf[k / kFctMaps], c->nx, c->nz, arrays[k % kFctMaps], width[k % kFctMaps]);
+  if (c->boxed && !c->dmaps) CK(cudaMalloc(&c->dmaps, sizeof c->hmaps), "cudaMalloc tensor maps");
   RunDesc* h = c->hdesc;
   h[0] = make_desc(c, 0, c->fct_tx, 0, 0);
   h[1] = make_desc(c, 1, c->fct_tx, 0, 0);
@@ -331,6 +380,7 @@ int flush_desc(ymkh_ctx* c, cudaStream_t s) {
   if (!c->desc_ok) { int rc = upload_desc(c); if (rc) return rc; }
   if (c->desc_pending) {
     CK(upload_table(c->ddesc, c->hdesc, sizeof c->hdesc, s), "upload run descriptors");
+    if (c->boxed) CK(upload_table(c->dmaps, c->hmaps, sizeof c->hmaps, s), "upload tensor maps");
     c->desc_pending = false;
   }
   return 0;
@@ -833,6 +883,7 @@ int ymkh_destroy(ymkh_ctx* c) {
   if (c->gpart) cudaFree(c->gpart);
   if (c->derr) cudaFree(c->derr);
   if (c->ddesc) cudaFree(c->ddesc);
+  if (c->dmaps) cudaFree(c->dmaps);
   if (c->xscratch) cudaFree(c->xscratch);
   delete c;
   return 0;
@@ -864,7 +915,7 @@ struct ymkh_batch {
   RunDesc* ddesc = nullptr;  // [2][cap]: tables for the members' current / next buffers
   int cap = 0;
   int fct_items = 0, mx_items = 0, fx_items = 0, fz_items = 0;
-  int tb = 64, fct_grid = 0, mx_grid = 0, fx_grid = 0, fz_grid = 0;
+  int tb = 128, fct_grid = 0, mx_grid = 0, fx_grid = 0, fz_grid = 0;
   int fct_mode = YMKH_FCT_FUSED;
   unsigned* derr = nullptr;
   bool dirty = true;
@@ -906,14 +957,17 @@ int batch_build(ymkh_batch* b, cudaStream_t s) {
       c->fct_mode = keep;
       if (rc) return rc;
     }
+    { int rc = flush_desc(c, s); if (rc) return rc; }  // the member's tensor maps
     RunDesc d0 = make_desc(c, c->cur, b->tb, f0, m0);
     RunDesc d1 = make_desc(c, 1 - c->cur, b->tb, f0, m0);
     d0.fx_item0 = d1.fx_item0 = x0;
     d0.fz_item0 = d1.fz_item0 = z0;
     x0 += items_fx(d0, c->nz);
     z0 += items_fz(d0, c->nz);
-    // batches take 128-row FCT segments round-robin (RunTable::fct_contig = 0)
-    d0.fct_seg = d1.fct_seg = std::min(c->nz, 128);
+    // one-row FCT segments in contiguous blocks, as a lone run's (at 16 uneven
+    // runs of 128..1024 x 256..2048, the step took 2422 us against 2453 with
+    // 128-row segments round-robin; at 24 runs of 64 x 768, 820 against 905)
+    d0.fct_seg = d1.fct_seg = kFctSegment;
     d0.mx_seg = d1.mx_seg = std::min(c->nz, 128);
     d0.fct_item0 = d1.fct_item0 = f0;
     d0.mx_item0 = d1.mx_item0 = m0;
@@ -941,7 +995,7 @@ int batch_build(ymkh_batch* b, cudaStream_t s) {
 int batch_step_once(ymkh_batch* b, cudaStream_t s) {
   const int n = (int)b->runs.size();
   if (!n) return 0;
-  RunTable T{b->ddesc + (size_t)b->parity * b->cap, n, b->fct_items, b->mx_items, b->derr, b->fx_items, b->fz_items, 0};
+  RunTable T{b->ddesc + (size_t)b->parity * b->cap, n, b->fct_items, b->mx_items, b->derr, b->fx_items, b->fz_items, 1};
   if (b->fct_mode == YMKH_FCT_SPLIT)
     CK(launch_fct_split_table(T, b->fx_grid, b->fz_grid, s), "fct_x/fct_z kernels (batch)");
   else

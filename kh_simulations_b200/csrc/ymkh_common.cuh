@@ -119,6 +119,24 @@ __device__ __forceinline__ void fct_nu_mu(double eps, double& nu, double& mu) {
   mu = 0.25 - 0.5 * nu;
 }
 
+// ux = px / n and vz = pz / n, the IEEE quotients, from one reciprocal
+// (div_rn).  Arguments outside the range where that is proven, other than a
+// zero momentum, take the division itself: momenta below 2^-800 (the quotient
+// must stay above 2^-900) or above 2^900, densities above 2^90.
+__device__ __forceinline__ bool velocity_range(double a) {
+  const unsigned h = (unsigned)__double2hiint(a) & 0x7fffffffu;
+  return h - ((1023u - 800u) << 20) < (1700u << 20) || (h | (unsigned)__double2loint(a)) == 0u;
+}
+__device__ __forceinline__ void velocities(double n, double px, double pz, double& ux, double& vz) {
+  const double y = __drcp_rn(n);
+  ux = div_rn(px, n, y);
+  vz = div_rn(pz, n, y);
+  if (!(velocity_range(px) && velocity_range(pz) && n < 0x1p90)) {
+    ux = px / n;
+    vz = pz / n;
+  }
+}
+
 // Periodic / clamped index maps of the shear axis (ymgpu2d/YM_FCT.cu:7-18 pad,
 // FCT_Sweeps.cu:68-81 clamped halo loads).
 __device__ __forceinline__ int xmap(int x, int nx, int periodic) {
@@ -240,6 +258,10 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes) {
   unsigned a = (unsigned)__cvta_generic_to_shared(bar);
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(a), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  unsigned a = (unsigned)__cvta_generic_to_shared(bar);
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a) : "memory");
+}
 // Spin on the phase with a bounded number of polls; on timeout the error
 // word is set and the caller carries on (the host reports it), so a lost
 // completion can never hang the GPU.
@@ -262,6 +284,27 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned by
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(d),
                "l"(src), "r"(bytes), "r"(b)
                : "memory");
+}
+constexpr int kFctMaps = 5;  // tensor maps of a state buffer: 128-wide boxes of 12, 9 and 1 arrays, 4-wide boxes of 12 and 9
+// A TMA tensor map as the kernels see it (128 opaque bytes, encoded on the host).
+struct alignas(64) TensorMap {
+  unsigned char bytes[128];
+};
+// Makes tensor maps written to global memory by the host visible to the TMA unit.
+__device__ __forceinline__ void tensormap_acquire(const TensorMap* m) {
+#pragma unroll
+  for (int k = 0; k < kFctMaps; ++k)
+    asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(m + k) : "memory");
+}
+// One box of a [array][z][x] tensor map to shared memory.  x must be even
+// (16-byte aligned), dst 128-byte aligned.
+__device__ __forceinline__ void box_g2s(void* dst, const TensorMap* map, int x, int z, int a, uint64_t* bar) {
+  unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  unsigned b = (unsigned)__cvta_generic_to_shared(bar);
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(d),
+      "l"(map), "r"(x), "r"(z), "r"(a), "r"(b)
+      : "memory");
 }
 // count doubles of a periodic row starting at shear index xs (which may be
 // negative or past the end), split at the wrap.  Requires nx even, xs even,
@@ -290,7 +333,8 @@ namespace ymkh {
 // kept).
 enum RowLoad : int {
   LOAD_ELEM = 0,    // per-element 8-byte cp.async through an x index table (walls, odd nx)
-  LOAD_BULK_ALL = 3 // TMA bulk row copies, one per thread spread over all warps
+  LOAD_BULK_ALL = 3, // TMA bulk row copies, one per thread spread over all warps
+  LOAD_BOX = 4       // FCT: evenly spaced arrays, a row is a few TMA boxes
 };
 
 // One run of a batch as the fused kernels see it: its start-of-step and
@@ -301,12 +345,13 @@ struct RunDesc {
   State in;
   State out;
   State xsw;  // x-swept fluid scratch of the split FCT form (fluid arrays only)
+  const TensorMap* maps;  // kFctMaps tensor maps of `in` (device memory; LOAD_BOX only)
   StepParams p;
   int fct_nstrips, fct_seg, fct_item0, fct_bulk;
   int mx_nstrips, mx_seg, mx_item0, mx_bulk;
   int fx_nstrips, fx_item0;           // split FCT, x pass: items (strip, row, beam)
   int fz_ncols, fz_seg, fz_item0;     // split FCT, z pass: items (column block, segment)
-  int pad_;
+  int pad_[1];
 };
 
 struct RunTable {
@@ -349,6 +394,7 @@ __device__ __forceinline__ void load_desc(RunDesc* dst, const RunDesc* src) {
 
 cudaError_t launch_fct_table(const RunTable& T, int tb, int grid_ctas, cudaStream_t s);
 cudaError_t launch_maxwell_table(const RunTable& T, int grid_ctas, cudaStream_t s);
+constexpr int kFctBoxWidth = 128;  // columns of the FCT's TMA boxes
 int fct_nstrips(int nx, int tb);
 int maxwell_nstrips(int nx);
 int fct_bulk_ok(const StepParams& p, int tb);

@@ -109,7 +109,7 @@ struct ZPipe {
 };
 
 template <int TB, int NST>
-__global__ void __launch_bounds__(4 * TB, (TB >= 128 ? 1 : 2))
+__global__ void __launch_bounds__(4 * TB, 2)
     fct_fused_kernel(const __grid_constant__ RunTable T) {
   constexpr int W = TB + 2;
   constexpr int NT = 4 * TB;
@@ -492,6 +492,585 @@ __global__ void __launch_bounds__(4 * TB, (TB >= 128 ? 1 : 2))
   }
 }
 
+// ---------------------------------------------------------------------------
+// The 128-wide form: one warp per swept variable.
+//
+// What bounds it: the FP64 and integer instructions of the 24 sweeps per cell,
+// at four warps a scheduler.  fct_fused_kernel issues 114 warp instructions a
+// cell: every phase of the x sweep goes through shared memory and a barrier,
+// each thread group forms its own velocities, and each row costs 33 row
+// copies.  Here a row costs 78:
+// - Twelve sweep warps take one variable of one beam each.  A lane owns four
+//   neighbouring columns, so most neighbours are its own registers and the
+//   rest come by shuffles; there is no barrier between the phases, and the
+//   four columns are independent work.
+// - Four coefficient warps run a row ahead: velocities, the interface
+//   coefficients of both directions and all sources, once per cell and beam
+//   (the field averages once for both beams), handed over in shared memory
+//   through mbarriers (co_full, co_free; two slots).
+// - A row arrives as three TMA boxes of 12, 12 and 9 arrays, requested by one
+//   thread four rows ahead (six more small ones where the window wraps).
+// - While every input is finite and far from overflow, the limiter needs two
+//   compares (fct_limit_fin); a row that is not sends the rest of the piece
+//   through the NaN-exact form.
+// - The sweep warps hold 72 registers of z history: setmaxnreg gives them 136
+//   and the coefficient warps 104 of the 512 x 128 at launch.
+// Measured (FCT, one step, against the 128-wide fct_fused_kernel): 3.42 ms
+// against 5.17 at 4096 x 8192, 251 us against 366 at 1024 x 2048.  Tried and
+// slower: the z history rotated through names by unrolling the row loop two or
+// three times (no register moves, but spills and a loop past the instruction
+// cache: 3.6 and 5.3 ms), separate fast and slow row loops, a CTA barrier per
+// row in place of the mbarriers, divisions in place of `velocities` (4% more).
+
+namespace {
+
+constexpr int F2_W = kFctBoxWidth;  // staged positions per row: position q holds shear index x0 - 4 + q
+constexpr int F2_O = 120;    // output columns per strip: positions 4 .. 123 (lanes 1 .. 30, four each)
+constexpr int F2_NT = 512;   // 12 sweep warps, 4 coefficient warps
+constexpr int F2_SWEEP = 12;
+constexpr int F2_NFL = 6;    // ring depth of the fluid rows
+constexpr int F2_NFD = 4;    // ring depth of the field rows, read by the coefficient warps only
+// field rows of a stage, in the state's array order: row z of Ex, Ez, By, Az,
+// row z-1 of Ez, By, Az, and n at z+1 and z-1 (warm_T only)
+constexpr int F2_EX = 0, F2_EZ = 3, F2_BY = 6, F2_AZ = 9, F2_EZM = 12, F2_BYM = 15, F2_AZM = 18, F2_NZP = 21, F2_NZM = 23;
+constexpr int F2_FD = 25;
+constexpr int F2_WRAP = 144;  // wrapped columns of a row: 33 arrays of 4 (in 128-byte aligned blocks of 12)
+
+// Rows a coefficient warp hands to the sweep warps, per beam: x-interface
+// 0.5*eps and nu, dt * px source; z-interface 0.5*eps and nu, mu of the
+// previous z-interface, dt * (pz, Q1..Q3 source) of the previous row.
+constexpr int HR_XH = 0, HR_XNU = 1, HR_XS = 2, HR_ZH = 3, HR_ZNU = 4, HR_ZMU = 5, HR_ZS = 6, HR_SIZE = 10;
+// Layout of such a row: position q at pair (q >> 1) of the even or odd
+// pairs, so that lane l's four positions are two 16-byte loads at stride 16
+// (no bank conflict) and the writers' 8-byte stores conflict-free too (the
+// odd pairs start 64 bytes past a 128-byte boundary).
+constexpr int HR_ODD = 72, HR_W = 136;
+__device__ __forceinline__ int hr_pos(int q) { return ((q >> 1) & 1) * HR_ODD + (q >> 2) * 2 + (q & 1); }
+
+__device__ __forceinline__ void ld4(double (&v)[4], const double* p0, const double* p1) {
+  const double2 a = *reinterpret_cast<const double2*>(p0), b = *reinterpret_cast<const double2*>(p1);
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+
+constexpr int F2_NCO = 2;  // coefficient slots
+static_assert(F2_NFL == 4 + F2_NCO && F2_NFD == 4, "row i+4 takes the fluid slot of row i-2 and the field slot of row i");
+
+// Barrier of the coefficient warps (id 1; 0 is __syncthreads).
+__device__ __forceinline__ void coef_bar() {
+  asm volatile("bar.sync 1, %0;" ::"n"(F2_NT - 32 * F2_SWEEP) : "memory");
+}
+
+// The limiter for finite arguments: the same result as fct_limit_sel.  With
+// s the sign of d0, max(0, min(s dm1, |f|, s dp1)) is zero when dm1 or dp1 has
+// the other sign, else the smallest of the three magnitudes; s then gives it
+// d0's sign.  Two compares instead of five, and no sign flips.
+__device__ __forceinline__ double fct_limit_fin(double f, double dm1, double d0, double dp1) {
+  const int h0 = __double2hiint(d0);
+  const int differ = (__double2hiint(dm1) ^ h0) | (__double2hiint(dp1) ^ h0);  // sign bit
+  double m = fabs(dp1) < fabs(dm1) ? dp1 : dm1;
+  m = fabs(f) < fabs(m) ? f : m;
+  const int lo = differ < 0 ? 0 : __double2loint(m);
+  const int hi = differ < 0 ? 0 : __double2hiint(m);
+  return __hiloint2double((hi & 0x7fffffff) | (h0 & (int)0x80000000), lo);
+}
+
+// Inputs below 2^100 and coefficients below 2^200 in magnitude keep every
+// product and sum of a sweep far from overflow (at most 2^800 or so).
+constexpr int F2_BIG_HI = (1023 + 100) << 20;
+constexpr double F2_BIG = 0x1p200;
+
+}  // namespace
+
+constexpr size_t fct_strip_smem_bytes() {
+  return sizeof(double) * ((size_t)F2_W * (F2_NFL * 12 + F2_NFD * F2_FD) + F2_NFD * F2_WRAP + F2_NCO * 2 * HR_SIZE * HR_W) +
+         sizeof(int) * F2_W + 8 * (F2_NFL + 2 * F2_NCO + 1) + sizeof(double) * (4 * F2_W + 2);
+}
+
+__global__ void __launch_bounds__(F2_NT, 1) fct_strip_kernel(const __grid_constant__ RunTable T) {
+  constexpr int W = F2_W;
+  constexpr unsigned FULL = 0xffffffffu;
+  extern __shared__ __align__(128) double strip_smem[];
+  double* const sfl = strip_smem;                              // [F2_NFL][12][W]
+  double* const sfd = sfl + (size_t)F2_NFL * 12 * W;     // [F2_NFD][F2_FD][W]
+  double* const wrap = sfd + (size_t)F2_NFD * F2_FD * W;  // [F2_NFD][F2_WRAP] wrapped columns
+  double* const hlp = wrap + F2_NFD * F2_WRAP;  // [F2_NCO][2 beams][HR_SIZE][HR_W]
+  int* const xtab = reinterpret_cast<int*>(hlp + F2_NCO * 2 * HR_SIZE * HR_W);
+  uint64_t* const bars = reinterpret_cast<uint64_t*>(xtab + W);  // row staged [F2_NFL]
+  uint64_t* const co_full = bars + F2_NFL;                        // coefficients written [F2_NCO]
+  uint64_t* const co_free = co_full + F2_NCO;                     // row and coefficients read [F2_NCO]
+  double* const uxr = reinterpret_cast<double*>(co_free + F2_NCO + 1);  // [2][2 beams][W] ux of the row
+
+  __shared__ RunDesc rd;
+  __shared__ int s_run, s_bad;
+  __shared__ RowCopy cpt[40];
+  const State& st = rd.in;
+  const State& out = rd.out;
+  const StepParams& p = rd.p;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+
+  if (tid == 0) {
+    for (int s = 0; s < F2_NFL; ++s) mbar_init(&bars[s], 1);
+    for (int s = 0; s < F2_NCO; ++s) {
+      mbar_init(&co_full[s], F2_NT / 32 - F2_SWEEP);
+      mbar_init(&co_free[s], F2_SWEEP);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  // sequence number of the piece's first row in the rings
+  unsigned seq = 0;
+  unsigned phase_bits = 0;  // per-barrier phase of the bulk path (one coefficient thread waits)
+
+  const bool contig = T.fct_contig != 0;
+  const int per = contig ? (T.fct_items + (int)gridDim.x - 1) / (int)gridDim.x : 0;
+  const int i_beg = contig ? (int)blockIdx.x * per : (int)blockIdx.x;
+  const int i_end = contig ? min(T.fct_items, i_beg + per) : T.fct_items;
+
+  // The piece that starts at an item: its run, strip and rows.  Every thread
+  // calls it once per piece; the barriers also end the previous piece.
+  struct Piece {
+    int x0, zs, ze, next;
+    bool warm, wall, bulk, box, edge;
+  };
+  auto begin_piece = [&](int item) -> Piece {
+    Piece c;
+    __syncthreads();  // previous piece fully consumed
+    if (tid == 0) {
+      s_run = find_run(T.runs, T.nruns, item, false);
+      s_bad = 0;
+    }
+    __syncthreads();
+    load_desc(&rd, &T.runs[s_run]);
+    __syncthreads();
+    const int nx = p.nx, nz = p.nz;
+    c.warm = p.warm_T > 0.0;
+    c.wall = !p.periodic_x;
+    c.bulk = rd.fct_bulk != LOAD_ELEM;
+    const int nseg = (nz + rd.fct_seg - 1) / rd.fct_seg;
+    const int local = item - rd.fct_item0;
+    int strip;
+    if (contig) {
+      strip = local / nseg;
+      const int seg0 = local - strip * nseg;
+      c.next = min(i_end, rd.fct_item0 + (strip + 1) * nseg);  // past this piece's last segment
+      c.zs = seg0 * rd.fct_seg;
+      c.ze = min(nz, (seg0 + (c.next - item)) * rd.fct_seg);
+    } else {
+      strip = local % rd.fct_nstrips;
+      c.zs = (local / rd.fct_nstrips) * rd.fct_seg;
+      c.ze = min(nz, c.zs + rd.fct_seg);
+      c.next = item + (int)gridDim.x;
+    }
+    c.x0 = strip * F2_O;
+    c.edge = c.x0 == 0 || c.x0 - 4 + W > nx;
+    c.box = rd.fct_bulk == LOAD_BOX && !(c.warm && c.edge);
+    return c;
+  };
+
+  if (warp < F2_SWEEP) {
+    // -------------------------------------------------- a sweep warp: one variable of one beam
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 136;");
+    const int beam = warp / 6, k = warp - beam * 6;
+    const bool has_sx = (k == FPX), has_sz = (k >= FPZ);
+    const double* const fl0 = sfl + (beam * 6 + k) * W + 4 * lane;
+    const double* const fl_last = fl0 + (size_t)(F2_NFL - 1) * 12 * W;
+    const double* const hlp0 = hlp + beam * (HR_SIZE * HR_W) + 2 * lane;
+    const double* fl = fl0;  // this lane's columns of the row, in the ring
+    unsigned gc = 0;         // rows read so far: coefficient slot and phase
+    for (int item = i_beg; item < i_end;) {
+      const Piece c = begin_piece(item);
+      item = c.next;
+      __syncthreads();  // the coefficient warps' row table
+      const int nx = p.nx;
+      const int nrow = c.ze - c.zs + 6;  // rows zs-3 .. ze+2
+      double* dst = (beam ? out.b[k] : out.a[k]) + idx2(0, c.zs, nx);
+      const int xo = c.x0 - 4 + 4 * lane;  // first of this lane's four columns
+      const bool owner = lane >= 1 && lane <= 30 && xo < nx;
+      const bool bulk = c.bulk;
+      const int wall_x = (c.wall && k == FPX) ? nx - 1 : -1;  // px is zero at x = 0 and here
+      double V1[4], f1[4], d1[4], L2[4], Na[4], Nb[4], Nc[4], A2[4], F3[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) V1[j] = f1[j] = d1[j] = L2[j] = Na[j] = Nb[j] = Nc[j] = A2[j] = F3[j] = 0.0;
+
+      // Whether every input of row i is finite and small enough that no
+      // later product or sum can overflow: then no NaN or infinity arises,
+      // and the limiter may use plain compares.
+      auto row_is_finite = [&] {
+        double v[4];
+        ld4(v, fl, fl + 2);
+        const int m = max(max(__double2hiint(v[0]) & 0x7fffffff, __double2hiint(v[1]) & 0x7fffffff),
+                          max(__double2hiint(v[2]) & 0x7fffffff, __double2hiint(v[3]) & 0x7fffffff));
+        return !__any_sync(FULL, m >= F2_BIG_HI) && *(volatile int*)&s_bad == 0;
+      };
+      // Row i: x sweep of the row, then one step of the z sweep down the
+      // lane's columns; N4, N3, N2 are the last three z lnrhot rows and N4
+      // receives the new one.
+      auto row = [&](bool fin, int i, double(&N4)[4], double(&N3)[4], double(&N2)[4]) {
+        const double* const hr = hlp0 + (gc & 1u) * (2 * HR_SIZE * HR_W);
+        // ---- x sweep (FCT_Sweeps.cu:88-162): interface j is between this lane's columns j and j+1
+        double ln[4], fx[4];
+        {
+          double v[4], h[4], nu[4], F[4], D[4], lo[4], dd[4];
+          ld4(v, fl, fl + 2);
+          ld4(h, hr + HR_XH * HR_W, hr + HR_XH * HR_W + HR_ODD);
+          ld4(nu, hr + HR_XNU * HR_W, hr + HR_XNU * HR_W + HR_ODD);
+          const double vr = __shfl_down_sync(FULL, v[0], 1);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const double vn = j < 3 ? v[j + 1] : vr;
+            F[j] = h[j] * (v[j] + vn);
+            D[j] = nu[j] * (vn - v[j]);
+          }
+          const double Fl = __shfl_up_sync(FULL, F[3], 1), Dl = __shfl_up_sync(FULL, D[3], 1);
+          if (has_sx) {
+            double s[4];
+            ld4(s, hr + HR_XS * HR_W, hr + HR_XS * HR_W + HR_ODD);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = v[j] + s[j];
+          }
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            lo[j] = v[j] - (F[j] - (j ? F[j - 1] : Fl));
+            ln[j] = lo[j] + (D[j] - (j ? D[j - 1] : Dl));
+          }
+          const double lor = __shfl_down_sync(FULL, lo[0], 1), lnr = __shfl_down_sync(FULL, ln[0], 1);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) dd[j] = (j < 3 ? ln[j + 1] : lnr) - ln[j];
+          const double ddl = __shfl_up_sync(FULL, dd[3], 1), ddr = __shfl_down_sync(FULL, dd[0], 1);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const double mu = fma(-0.5, nu[j], 0.25);  // 0.25 - 0.5*nu: 0.5*nu is exact
+            fx[j] = mu * ((j < 3 ? lo[j + 1] : lor) - lo[j]);
+          }
+          if (fin) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) fx[j] = fct_limit_fin(fx[j], j ? dd[j - 1] : ddl, dd[j], j < 3 ? dd[j + 1] : ddr);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) fx[j] = fct_limit_sel(fx[j], j ? dd[j - 1] : ddl, dd[j], j < 3 ? dd[j + 1] : ddr);
+          }
+        }
+        const double fxl = __shfl_up_sync(FULL, fx[3], 1);
+        // ---- z sweep: row i-3 leaves when row i arrives
+        double ov[4];
+        {
+          double h[4], nu[4], mu1[4], s[4];
+          ld4(h, hr + HR_ZH * HR_W, hr + HR_ZH * HR_W + HR_ODD);
+          ld4(nu, hr + HR_ZNU * HR_W, hr + HR_ZNU * HR_W + HR_ODD);
+          ld4(mu1, hr + HR_ZMU * HR_W, hr + HR_ZMU * HR_W + HR_ODD);
+          if (has_sz) ld4(s, hr + (HR_ZS + k - FPZ) * HR_W, hr + (HR_ZS + k - FPZ) * HR_W + HR_ODD);
+          double fl4[4], fad[4], lz[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const double Vx = ln[j] - (fx[j] - (j ? fx[j - 1] : fxl));
+            const double fR = h[j] * (V1[j] + Vx);
+            const double dR = nu[j] * (Vx - V1[j]);
+            const double vs = has_sz ? V1[j] + s[j] : V1[j];
+            const double lo = vs - (fR - f1[j]);
+            lz[j] = lo + (dR - d1[j]);
+            fad[j] = mu1[j] * (lo - L2[j]);
+            V1[j] = Vx;
+            f1[j] = fR;
+            d1[j] = dR;
+            L2[j] = lo;
+          }
+          if (fin) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) fl4[j] = fct_limit_fin(A2[j], N3[j] - N4[j], N2[j] - N3[j], lz[j] - N2[j]);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) fl4[j] = fct_limit_sel(A2[j], N3[j] - N4[j], N2[j] - N3[j], lz[j] - N2[j]);
+          }
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            ov[j] = N3[j] - (fl4[j] - F3[j]);
+            F3[j] = fl4[j];
+            A2[j] = fad[j];
+            N4[j] = lz[j];
+          }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&co_free[gc & 1u]);
+        ++gc;
+        fl = fl == fl_last ? fl0 : fl + 12 * W;
+        if (i >= 6) {  // row zs + i - 6 (YM_Fluid.cu:20-29: density floor, wall momentum)
+          if (k == FN) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              if (ov[j] < 0.05) ov[j] = 0.05;
+          }
+          if (owner && dbg_ok(xo >= 0 && c.zs + i - 6 < c.ze, T.err)) {
+            if (bulk) {  // nx even, rows 16-byte aligned
+              *reinterpret_cast<double2*>(dst + xo) = make_double2(ov[0], ov[1]);
+              if (xo + 2 < nx) *reinterpret_cast<double2*>(dst + xo + 2) = make_double2(ov[2], ov[3]);
+            } else {
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                if (xo + j < nx) dst[xo + j] = (wall_x >= 0 && (xo + j == 0 || xo + j == wall_x)) ? 0.0 : ov[j];
+            }
+          }
+          dst += nx;
+        }
+      };
+
+      // row i staged and its coefficients written / row i read
+      auto wait_row = [&] { mbar_wait(&co_full[gc & 1u], (gc >> 1) & 1u, T.err); };
+      bool fin = true;
+      for (int i = 0; i < nrow; ++i) {
+        wait_row();
+        if (fin) fin = row_is_finite();
+        row(fin, i, Na, Nb, Nc);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const double t = Na[j];
+          Na[j] = Nb[j];
+          Nb[j] = Nc[j];
+          Nc[j] = t;
+        }
+      }
+    }
+  } else {
+    // -------------------------------------------------- a coefficient warp: 32 positions, both beams
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 104;");
+    const int htid = tid - F2_SWEEP * 32;
+    const int q = htid;
+    const int hq = hr_pos(q);
+    unsigned gc = 0;        // rows handed over so far: coefficient slot and phase
+    int s6 = 0, s4 = 0;     // ring slots of the next row
+    const int q_next = q < W - 1 ? 1 : 0;  // the last position has no interface
+    for (int item = i_beg; item < i_end;) {
+      const Piece c = begin_piece(item);
+      item = c.next;
+      const int nx = p.nx, nz = p.nz, x0 = c.x0;
+      const bool warm = c.warm, bulk = c.bulk, box = c.box;
+      const int narr = 33 + (warm ? 4 : 0);
+      // Evenly spaced arrays (box): a row is three TMA boxes (and four for
+      // warm_T).  Past the edges of the grid they read zeros, so where the
+      // window wraps, the four wrapped columns next to the edge (all that the
+      // strip's outputs need: those before x = 0 in the first strip, from
+      // x = nx in the last) come as three narrow boxes and are put in their
+      // places when the row is there.  With warm_T such a strip copies row by row.
+      const TensorMap* const maps = rd.maps;  // boxes of 12, 9 and 1 arrays; 4-wide boxes of 12 and 9 arrays
+      if (box && htid == 0) tensormap_acquire(maps);
+      const bool patch_l = x0 == 0, patch = box && c.edge;
+      const int patch_q = patch_l ? 0 : nx - (x0 - 4);  // position of the first wrapped column
+      if (!bulk) xtab[q] = xmap(x0 - 4 + q, nx, p.periodic_x);
+      // row copies of the piece: source array, its row (z, z-1, z+1), its place in the fluid or field ring
+      if (htid < narr) {
+        const int a = htid;
+        const double* base;
+        int dst, kind_row = 0;
+        if (a < 12) {
+          base = a < 6 ? st.a[a] : st.b[a - 6];
+          dst = a;
+        } else if (a < 33) {  // fields 0..11 of row z, 3..11 of row z-1
+          dst = a - 12;
+          base = st.f[dst < 12 ? dst : dst - 9];
+          kind_row = dst < 12 ? 0 : 1;
+        } else {
+          const int w = a - 33;  // n at z+1 (A, B), n at z-1 (A, B)
+          base = (w & 1) ? st.b[FN] : st.a[FN];
+          dst = F2_NZP + w;
+          kind_row = (w >> 1) ? 1 : 2;
+        }
+        int x = (x0 - 4) % nx;
+        x = x < 0 ? x + nx : x;
+        cpt[a].base = base + x;
+        cpt[a].base0 = base;
+        cpt[a].dst = dst;
+        cpt[a].kind = kind_row;
+        cpt[a].len1 = min(W, nx - x);
+      }
+      __syncthreads();
+      const int r_first = c.zs - 3;
+      const int nrow = c.ze - c.zs + 6;
+
+      // requests row i of the piece (coefficient warps only)
+      auto issue_row = [&](int i) {
+        const unsigned g = seq + (unsigned)i;
+        double* const fl = sfl + (size_t)(g % F2_NFL) * 12 * W;
+        double* const fd = sfd + (size_t)(g % F2_NFD) * F2_FD * W;
+        uint64_t* const bar = &bars[g % F2_NFL];
+        const int zr = zclamp(r_first + i, nz);
+        const int zm = (zr == 0) ? nz - 1 : zr - 1;
+        const int zp = (zr == nz - 1) ? 0 : zr + 1;
+        const bool rows_ok = dbg_ok(zr >= 0 && zr < nz && zm >= 0 && zm < nz && zp >= 0 && zp < nz, T.err);
+        if (box) {
+          if (htid == 0) {
+            mbar_expect_tx(bar, (unsigned)((narr * W + (patch ? 33 * 4 : 0)) * 8));
+            if (rows_ok) {
+              if (patch) {
+                double* const wr = wrap + (g % F2_NFD) * F2_WRAP;
+                const int xw = patch_l ? nx - 4 : 0;
+                box_g2s(wr, maps + 3, xw, zr, 12, bar);
+                box_g2s(wr + 48, maps + 3, xw, zr, 0, bar);
+                box_g2s(wr + 96, maps + 4, xw, zm, 3, bar);
+              }
+              box_g2s(fl, maps, x0 - 4, zr, 12, bar);
+              box_g2s(fd, maps, x0 - 4, zr, 0, bar);
+              box_g2s(fd + F2_EZM * W, maps + 1, x0 - 4, zm, 3, bar);
+              if (warm) {
+                box_g2s(fd + F2_NZP * W, maps + 2, x0 - 4, zp, 12, bar);
+                box_g2s(fd + (F2_NZP + 1) * W, maps + 2, x0 - 4, zp, 18, bar);
+                box_g2s(fd + F2_NZM * W, maps + 2, x0 - 4, zm, 12, bar);
+                box_g2s(fd + (F2_NZM + 1) * W, maps + 2, x0 - 4, zm, 18, bar);
+              }
+            }
+          }
+        } else if (bulk) {
+          // one row copy per thread, spread over the warps (lane-major)
+          if (htid == 0) mbar_expect_tx(bar, (unsigned)(narr * W * 8));
+          const int ca = lane * (F2_NT / 32 - F2_SWEEP) + warp - F2_SWEEP;
+          if (ca < narr) {
+            const RowCopy& c = cpt[ca];
+            const int len1 = c.len1;
+            if (rows_ok && dbg_ok(len1 > 0 && c.dst >= 0 && c.dst < (ca < 12 ? 12 : F2_FD), T.err)) {
+              const size_t off = (size_t)(c.kind == 0 ? zr : (c.kind == 1 ? zm : zp)) * nx;
+              double* const dst = (ca < 12 ? fl : fd) + c.dst * W;
+              bulk_g2s(dst, c.base + off, (unsigned)len1 * 8u, bar);
+              for (int done = len1; done < W;) {  // past the periodic wrap (more than once if nx < W)
+                const int len = min(W - done, nx);
+                bulk_g2s(dst + done, c.base0 + off, (unsigned)len * 8u, bar);
+                done += len;
+              }
+            }
+          }
+        } else {
+          const int x = xtab[htid];
+          if (rows_ok && dbg_ok(x >= 0 && x < nx, T.err))
+            for (int a = 0; a < narr; ++a) {
+              const RowCopy& c = cpt[a];
+              const size_t off = (size_t)(c.kind == 0 ? zr : (c.kind == 1 ? zm : zp)) * nx;
+              cp_async8((a < 12 ? fl : fd) + c.dst * W + htid, c.base0 + off + x);
+            }
+          cp_async_commit();
+        }
+      };
+
+      int ps = q;  // at a wall the clamped ghost cells carry the edge cell's px source
+      if (c.wall) {
+        const int xg = x0 - 4 + q;
+        ps = (xg < 0 ? 0 : (xg >= nx ? nx - 1 : xg)) - (x0 - 4);
+      }
+      ps = max(1, min(W - 2, ps));  // positions 0 and 127 are not used
+      const double dt = p.dt;
+      const double dtdx = p.dt / p.dx;
+      const double dtdz = p.dt / p.dz;
+      double U1[2] = {0.0, 0.0}, mu1[2] = {0.0, 0.0}, S1[2][4];
+#pragma unroll
+      for (int b = 0; b < 2; ++b) S1[b][0] = S1[b][1] = S1[b][2] = S1[b][3] = 0.0;
+      for (int i = 0; i < 4; ++i)
+        if (i < nrow) issue_row(i);
+        else if (!bulk) cp_async_commit();
+      // element e of the wrapped columns: column e & 3 of array e >> 2
+      auto patch_row = [&](double* fl, double* fd, const double* src) {
+        for (int e = htid; e < 33 * 4; e += W) {
+          const int a = e >> 2, x = patch_q + (e & 3);
+          if (x < W) (a < 12 ? fl + a * W : fd + (a - 12) * W)[x] = src[e];
+        }
+      };
+      for (int i = 0; i < nrow; ++i) {
+        // row i staged
+        if (bulk) {
+          const unsigned b = (seq + (unsigned)i) % F2_NFL;
+          mbar_wait(&bars[b], (phase_bits >> b) & 1u, T.err);
+          phase_bits ^= 1u << b;
+        } else {
+          cp_async_wait<3>();
+          coef_bar();
+        }
+        if (patch) {
+          patch_row(sfl + s6 * (12 * W), sfd + s4 * (F2_FD * W), wrap + s4 * F2_WRAP);
+          coef_bar();
+        }
+        const double* const fl = sfl + s6 * (12 * W) + q;
+        const double* const fd = sfd + s4 * (F2_FD * W) + ps;
+        s6 = s6 == F2_NFL - 1 ? 0 : s6 + 1;
+        s4 = (s4 + 1) & (F2_NFD - 1);
+        double* const ur = uxr + (gc & 1u) * (2 * W) + q;
+        double* const hr0 = hlp + (gc & 1u) * (2 * HR_SIZE * HR_W) + hq;
+        // velocities (YM_Fluid.cu:3-11); the x interface also needs the next position's
+        double ux[2], vz[2];
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+          velocities(max_sel(fl[(b * 6 + FN) * W], 0.05), fl[(b * 6 + FPX) * W], fl[(b * 6 + FPZ) * W], ux[b], vz[b]);
+          ur[b * W] = ux[b];
+        }
+        // field averages at the cell, shared by both beams (YM_Fluid.cu:43-66, 99-102)
+        double ex[3], by[3], ez[3], az[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const double* e = fd + c * W;
+          ex[c] = 0.5 * (e[F2_EX * W] + e[F2_EX * W - 1]);
+          by[c] = 0.25 * (e[F2_BY * W] + e[F2_BY * W - 1] + e[F2_BYM * W] + e[F2_BYM * W - 1]);
+          ez[c] = 0.5 * (e[F2_EZ * W] + e[F2_EZM * W]);
+          az[c] = 0.5 * (e[F2_AZ * W] + e[F2_AZM * W]);
+        }
+        double sx[2], sz[2], sq[2][3];
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+          const double q1 = fl[(b * 6 + FQ1) * W], q2 = fl[(b * 6 + FQ2) * W], q3 = fl[(b * 6 + FQ3) * W];
+          sx[b] = -(q1 * (ex[0] + vz[b] * by[0]) + q2 * (ex[1] + vz[b] * by[1]) + q3 * (ex[2] + vz[b] * by[2]));
+          sz[b] = -(q1 * (ez[0] - ux[b] * by[0]) + q2 * (ez[1] - ux[b] * by[1]) + q3 * (ez[2] - ux[b] * by[2]));
+          const double av = p.alpha * vz[b];  // YM_Fluid.cu:103-107
+          sq[b][0] = dt * (av * (q2 * az[2] - q3 * az[1]));
+          sq[b][1] = dt * (av * (q3 * az[0] - q1 * az[2]));
+          sq[b][2] = dt * (av * (q1 * az[1] - q2 * az[0]));
+        }
+        if (warm) {  // YM_Fluid.cu:71-80
+#pragma unroll
+          for (int b = 0; b < 2; ++b) {
+            const double* nn = fl + (b * 6 + FN) * W + (ps - q);
+            const double* nz_ = fd + (q - ps) + b * W;
+            sx[b] -= p.warm_T * ((nn[1] - nn[-1]) / (2.0 * p.dx));
+            sz[b] -= p.warm_T * ((nz_[F2_NZP * W] - nz_[F2_NZM * W]) / (2.0 * p.dz));
+          }
+        }
+        coef_bar();  // every position's ux written, the row's fields read: its field slot is free
+        // the coefficient slot free: every sweep warp is past row i-2, whose fluid slot row i+4 takes
+        mbar_wait(&co_free[gc & 1u], ((gc >> 1) & 1u) ^ 1u, T.err);
+        if (i + 4 < nrow) issue_row(i + 4);
+        else if (!bulk) cp_async_commit();
+        double size = 0.0;  // of everything handed to the sweep warps
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+          double* const hr = hr0 + b * (HR_SIZE * HR_W);
+          const double e = fct_eps(ux[b], ur[b * W + q_next], dtdx);
+          double nu, mu;
+          fct_nu_mu(e, nu, mu);
+          hr[HR_XH * HR_W] = 0.5 * e;
+          hr[HR_XNU * HR_W] = nu;
+          size += nu;
+          const double ezi = fct_eps(U1[b], vz[b], dtdz);
+          fct_nu_mu(ezi, nu, mu);
+          hr[HR_ZH * HR_W] = 0.5 * ezi;
+          hr[HR_ZNU * HR_W] = nu;
+          hr[HR_ZMU * HR_W] = mu1[b];
+          size += nu;
+          U1[b] = vz[b];
+          mu1[b] = mu;
+          sx[b] = dt * sx[b];
+          sz[b] = dt * sz[b];
+          hr[HR_XS * HR_W] = sx[b];
+#pragma unroll
+          for (int v = 0; v < 4; ++v) hr[(HR_ZS + v) * HR_W] = S1[b][v];
+          S1[b][0] = sz[b];
+          S1[b][1] = sq[b][0];
+          S1[b][2] = sq[b][1];
+          S1[b][3] = sq[b][2];
+          size += fabs(sx[b]) + fabs(sz[b]);
+          size += (fabs(sq[b][0]) + fabs(sq[b][1])) + fabs(sq[b][2]);
+        }
+        if (!(size < F2_BIG)) s_bad = 1;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&co_full[gc & 1u]);
+        ++gc;
+      }
+      if (!bulk) cp_async_wait<0>();
+      seq += (unsigned)nrow;
+    }
+  }
+}
+
 template <int TB, int NST>
 static cudaError_t prepare_fct_t() {
   return cudaFuncSetAttribute(fct_fused_kernel<TB, NST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -507,9 +1086,14 @@ constexpr int fct_nst() {
   return 4;
 }
 
-int fct_nstrips(int nx, int tb) { return (nx + (tb - 6) - 1) / (tb - 6); }
+int fct_nstrips(int nx, int tb) {
+  const int out = tb == 128 ? F2_O : tb - 6;
+  return (nx + out - 1) / out;
+}
 
-int fct_bulk_ok(const StepParams& p, int tb) { return (p.periodic_x && (p.nx % 2) == 0 && p.nx >= tb + 2) ? 1 : 0; }
+int fct_bulk_ok(const StepParams& p, int tb) {
+  return (p.periodic_x && (p.nx % 2) == 0 && (tb == 128 || p.nx >= tb + 2)) ? 1 : 0;
+}
 
 // The kernel reads start-of-step values across strip and segment halos while
 // other CTAs write theirs, so each run's fluid goes to its second buffer
@@ -520,7 +1104,7 @@ cudaError_t launch_fct_table(const RunTable& T, int tb, int grid_ctas, cudaStrea
   switch (tb) {
     case 32: fct_fused_kernel<32, fct_nst<32>()><<<grid, 128, fct_smem_bytes<32>(fct_nst<32>()), s>>>(T); break;
     case 64: fct_fused_kernel<64, fct_nst<64>()><<<grid, 256, fct_smem_bytes<64>(fct_nst<64>()), s>>>(T); break;
-    case 128: fct_fused_kernel<128, fct_nst<128>()><<<grid, 512, fct_smem_bytes<128>(fct_nst<128>()), s>>>(T); break;
+    case 128: fct_strip_kernel<<<grid, F2_NT, fct_strip_smem_bytes(), s>>>(T); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
@@ -530,7 +1114,8 @@ cudaError_t prepare_fct(int tb) {
   switch (tb) {
     case 32: return prepare_fct_t<32, fct_nst<32>()>();
     case 64: return prepare_fct_t<64, fct_nst<64>()>();
-    case 128: return prepare_fct_t<128, fct_nst<128>()>();
+    case 128:
+      return cudaFuncSetAttribute(fct_strip_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fct_strip_smem_bytes());
     default: return cudaErrorInvalidValue;
   }
 }
@@ -540,7 +1125,7 @@ int fct_ctas_per_sm(int tb) {
   switch (tb) {
     case 32: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fct_fused_kernel<32, fct_nst<32>()>, 128, fct_smem_bytes<32>(fct_nst<32>())); break;
     case 64: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fct_fused_kernel<64, fct_nst<64>()>, 256, fct_smem_bytes<64>(fct_nst<64>())); break;
-    case 128: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fct_fused_kernel<128, fct_nst<128>()>, 512, fct_smem_bytes<128>(fct_nst<128>())); break;
+    case 128: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fct_strip_kernel, F2_NT, fct_strip_smem_bytes()); break;
     default: break;
   }
   return n;
