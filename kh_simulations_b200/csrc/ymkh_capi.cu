@@ -218,20 +218,32 @@ int setup_params(ymkh_ctx* c, const ymkh_params* p) {
   return 0;
 }
 
-// Segment length for persistent CTAs taking (strip, segment) items
-// round-robin: the smallest per-CTA item count whose last round is nearly
-// full, with segments of at least 16 rows.
-int pick_segment(int nz, int nstrips, int grid) {
-  int best_seg = nz, best_cost = 1 << 30;
-  for (int nseg = 1; nseg <= std::max(1, nz / 16); ++nseg) {
-    const int seg = (nz + nseg - 1) / nseg;
-    const int items = nstrips * ((nz + seg - 1) / seg);
-    const int rounds = (items + grid - 1) / grid;
-    // cost in rows per CTA, each item paying its 6-row start-up
-    const int cost = rounds * (seg + 6);
-    if (cost < best_cost) { best_cost = cost; best_seg = seg; }
+// Maxwell's segment rows for persistent CTAs taking (strip, segment) items
+// round-robin: the length whose busiest CTA has the least to do, each item
+// paying kMxStart rows of start-up besides its own (two rows staged ahead, the
+// pipeline's fill and the item's set-up; 2, 4 and 8 measured alike).  A row
+// costs a CTA about 2 us whatever the grid, so short segments over every SM
+// are what a small grid needs: against segments of at least 16 rows, 64 x 96
+// took 13 us instead of 49, 256 x 512 21 instead of 37; against 128 rows in
+// batches, 16 uneven runs 2.20 ms a step instead of 2.42.
+constexpr int kMxStart = 4;
+struct MxGrid {
+  int nz, nstrips;
+};
+int pick_mx_segment(const MxGrid* g, int n, int grid) {
+  int nz_max = 1;
+  for (int i = 0; i < n; ++i) nz_max = std::max(nz_max, g[i].nz);
+  int best = 1;
+  long long best_cost = 1ll << 60;
+  for (int nseg = 1; nseg <= nz_max; ++nseg) {
+    const int seg = (nz_max + nseg - 1) / nseg;
+    if (nseg > 1 && seg == (nz_max + nseg - 2) / (nseg - 1)) continue;
+    long long items = 0;
+    for (int i = 0; i < n; ++i) items += (long long)g[i].nstrips * ((g[i].nz + seg - 1) / seg);
+    const long long rounds = (items + grid - 1) / grid, cost = rounds * (seg + kMxStart);
+    if (cost < best_cost) { best_cost = cost; best = seg; }
   }
-  return best_seg;
+  return best;
 }
 
 // One-row segments: a CTA's contiguous block then ends at any row, so the
@@ -258,7 +270,8 @@ void choose_launch_shape(ymkh_ctx* c) {
   c->fct_seg = std::min(c->nz, kFctSegment);
   const int mx_per_sm = std::max(1, maxwell_ctas_per_sm());
   c->mx_grid = c->sms * mx_per_sm;
-  c->mx_seg = pick_segment(c->nz, maxwell_nstrips(c->nx), c->mx_grid);
+  const MxGrid mg{c->nz, maxwell_nstrips(c->nx)};
+  c->mx_seg = pick_mx_segment(&mg, 1, c->mx_grid);
   c->fx_grid = c->sms * std::max(1, fct_split_ctas_per_sm(0)) * 4;
   c->fz_grid = c->sms * std::max(1, fct_split_ctas_per_sm(1)) * 4;
 }
@@ -947,6 +960,9 @@ int batch_build(ymkh_batch* b, cudaStream_t s) {
     CK(cudaMalloc(&b->ddesc, 2 * (size_t)b->cap * sizeof(RunDesc)), "cudaMalloc batch descriptors");
   }
   std::vector<RunDesc> h(2 * (size_t)std::max(n, 1));
+  std::vector<MxGrid> mg;
+  for (const ymkh_ctx* c : b->runs) mg.push_back({c->nz, maxwell_nstrips(c->nx)});
+  const int mx_seg = pick_mx_segment(mg.data(), n, b->mx_grid);
   int f0 = 0, m0 = 0, x0 = 0, z0 = 0;
   for (int i = 0; i < n; ++i) {
     ymkh_ctx* c = b->runs[i];
@@ -968,7 +984,7 @@ int batch_build(ymkh_batch* b, cudaStream_t s) {
     // runs of 128..1024 x 256..2048, the step took 2422 us against 2453 with
     // 128-row segments round-robin; at 24 runs of 64 x 768, 820 against 905)
     d0.fct_seg = d1.fct_seg = kFctSegment;
-    d0.mx_seg = d1.mx_seg = std::min(c->nz, 128);
+    d0.mx_seg = d1.mx_seg = std::min(c->nz, mx_seg);
     d0.fct_item0 = d1.fct_item0 = f0;
     d0.mx_item0 = d1.mx_item0 = m0;
     h[i] = d0;
