@@ -315,190 +315,204 @@ cudaError_t prepare_column(int nz) {
 // Products and sums are rounded separately (no fused multiply-add), as the
 // reference's -fmad=false build rounds them.
 
+// Bound by the FP64 pipe: 4 operations per row, coefficient and column, none of
+// them fused, so 2.77 ms at 1024 x 2048 with 18 arrays and modes 342..512.
+// Both kernels keep the operand that belongs to a thread's columns in
+// registers (32 rows x 2 columns of the array; 16 x 2 running sums) and read
+// the twiddles, which all lanes share, as one 16-byte (cos, sin) load.  That
+// load takes two shared-memory cycles: with one column a thread it could only
+// feed four FP64 instructions and set the pace (81% of the load pipe, FP64
+// 70%); with two, eight.  Measured there: 1.88 + 1.72 ms at 78% of the FP64
+// pipe each, against 4.58 ms for the two kernels that loaded both operands of
+// a 2 x 4 and a 4 x 4 block from shared memory; 512 x 1024 0.53 against 0.65
+// ms.  Staging the coefficients in shared memory too cost the apply kernel a
+// CTA per SM (2.28 ms).
+//
 // The reference's warp reduction (shfl_down by 16, 8, 4, 2, 1) leaves lane 0
 // with root = T4(0) + T4(1), T4(i) = T3(i) + T3(i+2), T3(i) = T2(i) + T2(i+4),
 // T2(i) = T1(i) + T1(i+8), T1(i) = a_i + a_{i+16} (every sum is commutative,
 // so only the grouping matters).  Visited in bit-reversed order (0, 8, 4,
 // 12, 2, ...), the sixteen T1 nodes form a balanced pairwise tree over
 // consecutive visits, which a stack of four partial sums evaluates.
-__host__ __device__ constexpr int bitrev4(int k) {
-  return ((k & 1) << 3) | ((k & 2) << 1) | ((k & 4) >> 1) | ((k & 8) >> 3);
+constexpr int BD_TX = 128;    // columns per CTA
+constexpr int BD_CH = 32;     // z rows in registers: a warp of the reference
+constexpr int BC_NC = 2, BC_NT = BD_TX / BC_NC;  // coefficients: columns threadIdx.x + n * BC_NT per thread
+constexpr int BC_BM = 16;     // most modes of a coefficient CTA
+constexpr int BA_BM = 16;     // modes per twiddle tile of the apply kernel
+
+// Stages the twiddles of rows [z0, z0 + 32) and modes [m0, m0 + bm) as
+// tw[z][bm] (cos, sin) pairs, zero past the last row or mode.
+template <int NT>
+__device__ __forceinline__ void stage_twiddles(double2* tw, const double* __restrict__ W, int ldw, int z0, int m0, int bm,
+                                               int nz, int M) {
+  for (int i = threadIdx.x; i < BD_CH * bm; i += NT) {
+    const int z = i / bm, m = i - z * bm;
+    if (z0 + z < nz && m0 + m < M) cp_async16(&tw[i], W + (size_t)(z0 + z) * ldw + 2 * (m0 + m));
+    else tw[i] = make_double2(0.0, 0.0);
+  }
+  cp_async_commit();
 }
 
-constexpr int BC_TJ = 32, BC_TX = 64, BC_CH = 32;  // coefficient tile: 32 j (16 modes) x 64 columns, z chunks of 32
-constexpr int BC_RJ = 2, BC_RX = 4;                // per thread: one mode's (cos, sin) x 4 columns
-constexpr int BC_THREADS = (BC_TJ / BC_RJ) * (BC_TX / BC_RX);  // 256
-
-__global__ void __launch_bounds__(BC_THREADS, 2)
-    band_coef_kernel(const __grid_constant__ ArrayList arrs, const double* __restrict__ W, int ldw, int J,
+// C[2m + {0, 1}][x] for modes [m0, m0 + bm) of one array: the running sums of
+// the block's modes stay in shared memory, each thread's own.
+__global__ void __launch_bounds__(BC_NT)
+    band_coef_kernel(const __grid_constant__ ArrayList arrs, const double* __restrict__ W, int ldw, int M, int bm,
                      double* __restrict__ C, int nx, int nz, double inv2) {
-  __shared__ __align__(16) double sW[2][BC_CH][BC_TJ];  // [z][j]
-  __shared__ __align__(16) double sF[2][BC_CH][BC_TX];  // [z][x]
-  const int j0 = blockIdx.x * BC_TJ, x0 = blockIdx.y * BC_TX, k = blockIdx.z;
-  const double* G = arrs.p[k];
-  double* Ck = C + (size_t)k * J * nx;
-  const int tj = threadIdx.x % (BC_TJ / BC_RJ);  // mode of the tile
-  const int tx = threadIdx.x / (BC_TJ / BC_RJ);  // group of 4 columns
-  const int nch = (nz + BC_CH - 1) / BC_CH;
-
-  auto stage = [&](int buf, int ch) {
-    // 32 z rows of W (32 j) and of the array (64 x), asynchronously (8-byte
-    // cp.async; zero padding past the edges written directly), one commit
-    // group per chunk
-    for (int i = threadIdx.x; i < BC_CH * BC_TJ; i += BC_THREADS) {
-      const int zz = i / BC_TJ, c = i - zz * BC_TJ, z = ch * BC_CH + zz;
-      if (z < nz && j0 + c < J) cp_async8(&sW[buf][zz][c], W + (size_t)z * ldw + j0 + c);
-      else sW[buf][zz][c] = 0.0;
-    }
-    for (int i = threadIdx.x; i < BC_CH * BC_TX; i += BC_THREADS) {
-      const int zz = i / BC_TX, c = i - zz * BC_TX, z = ch * BC_CH + zz;
-      if (z < nz && x0 + c < nx) cp_async8(&sF[buf][zz][c], G + idx2(x0 + c, z, nx));
-      else sF[buf][zz][c] = 0.0;
-    }
-    cp_async_commit();
-  };
-
-  double S[BC_RJ][BC_RX];
+  constexpr int NC = BC_NC, NT = BC_NT;
+  extern __shared__ __align__(16) double2 band_smem[];
+  double2* const tw = band_smem;                                              // [2][BD_CH][bm]
+  double2* const sum = band_smem + (size_t)2 * BD_CH * bm + threadIdx.x;      // [bm][BD_TX]
+  const int m0 = blockIdx.x * bm, x0 = blockIdx.y * BD_TX + threadIdx.x, k = blockIdx.z;
+  const double* g = arrs.p[k] + x0;
+  bool in[NC];
 #pragma unroll
-  for (int a = 0; a < BC_RJ; ++a)
+  for (int n = 0; n < NC; ++n) in[n] = x0 + n * NT < nx;
+  const int nm = min(bm, M - m0), nch = (nz + BD_CH - 1) / BD_CH;
+  for (int m = 0; m < nm; ++m)
 #pragma unroll
-    for (int b = 0; b < BC_RX; ++b) S[a][b] = 0.0;
-
-  stage(0, 0);
+    for (int n = 0; n < NC; ++n) sum[m * BD_TX + n * NT] = make_double2(0.0, 0.0);
+  stage_twiddles<NT>(tw, W, ldw, 0, m0, bm, nz, M);
   for (int ch = 0; ch < nch; ++ch) {
-    const int buf = ch & 1;
-    // the next chunk goes to the other buffer, released by the barrier at
-    // the end of the previous chunk; then this chunk's copies are awaited
-    if (ch + 1 < nch) stage(buf ^ 1, ch + 1);
-    else cp_async_commit();
-    cp_async_wait<1>();
-    __syncthreads();
-    double st[4][BC_RJ][BC_RX];  // pending tree nodes of heights 1..4 (T2..T4 partial sums)
+    double f[NC][BD_CH];
 #pragma unroll
-    for (int kk = 0; kk < 16; ++kk) {
-      const int i = bitrev4(kk);
-      double w0[BC_RJ], w1[BC_RJ], f0[BC_RX], f1[BC_RX];
+    for (int i = 0; i < BD_CH; ++i)
 #pragma unroll
-      for (int a = 0; a < BC_RJ; ++a) {
-        w0[a] = sW[buf][i][tj * BC_RJ + a];
-        w1[a] = sW[buf][i + 16][tj * BC_RJ + a];
+      for (int n = 0; n < NC; ++n) {
+        const int z = ch * BD_CH + i;
+        f[n][i] = (in[n] && z < nz) ? g[(size_t)z * nx + n * NT] : 0.0;
       }
+    cp_async_wait<0>();
+    __syncthreads();  // this chunk's twiddles are there, the other buffer is free
+    if (ch + 1 < nch) stage_twiddles<NT>(tw + ((ch + 1) & 1) * BD_CH * bm, W, ldw, (ch + 1) * BD_CH, m0, bm, nz, M);
+    const double2* t = tw + (ch & 1) * BD_CH * bm;
+    for (int m = 0; m < nm; ++m, ++t) {
+      double sc[NC][4], ss[NC][4];  // pending tree nodes of heights 1..4 (T2..T4 partial sums)
 #pragma unroll
-      for (int b = 0; b < BC_RX; ++b) {
-        f0[b] = sF[buf][i][tx * BC_RX + b];
-        f1[b] = sF[buf][i + 16][tx * BC_RX + b];
-      }
+      for (int kk = 0; kk < 16; ++kk) {
+        const int i = bitrev4(kk);
+        const double2 w0 = t[i * bm], w1 = t[(i + 16) * bm];
 #pragma unroll
-      for (int a = 0; a < BC_RJ; ++a)
-#pragma unroll
-        for (int b = 0; b < BC_RX; ++b) {
-          const double p0 = f0[b] * w0[a];  // YM_Physics.cu:394 ar = v * cz (rounded)
-          const double p1 = f1[b] * w1[a];
-          double x = p0 + p1;  // T1(i)
-          // merge with the pending nodes: one level per trailing one bit of kk
-          int lvl = 0;
+        for (int n = 0; n < NC; ++n) {
+          double c = f[n][i] * w0.x + f[n][i + 16] * w1.x;  // T1(i); products rounded (YM_Physics.cu:394)
+          double s = f[n][i] * w0.y + f[n][i + 16] * w1.y;
+          int lvl = 0;  // merge with the pending nodes: one level per trailing one bit of kk
 #pragma unroll
           for (int L = 0; L < 4; ++L) {
             if (((kk >> L) & 1) && lvl == L) {
-              x = st[L][a][b] + x;
+              c = sc[n][L] + c;
+              s = ss[n][L] + s;
               ++lvl;
             }
           }
-          if (lvl < 4) st[lvl][a][b] = x;
-          else S[a][b] = S[a][b] + x;  // warp sums added in warp order from 0.0
+          if (lvl < 4) {
+            sc[n][lvl] = c;
+            ss[n][lvl] = s;
+          } else {  // warp sums added in warp order from 0.0
+            double2 S = sum[m * BD_TX + n * NT];
+            S.x = S.x + c;
+            S.y = S.y + s;
+            sum[m * BD_TX + n * NT] = S;
+          }
         }
+      }
     }
-    __syncthreads();
   }
+  double* Ck = C + (size_t)k * 2 * M * nx + (size_t)2 * m0 * nx + x0;
 #pragma unroll
-  for (int a = 0; a < BC_RJ; ++a)
-#pragma unroll
-    for (int b = 0; b < BC_RX; ++b) {
-      const int j = j0 + tj * BC_RJ + a, x = x0 + tx * BC_RX + b;
-      if (j < J && x < nx) Ck[(size_t)j * nx + x] = S[a][b] * inv2;
-    }
+  for (int n = 0; n < NC; ++n)
+    if (in[n])
+      for (int m = 0; m < nm; ++m) {
+        const double2 S = sum[m * BD_TX + n * NT];
+        Ck[(size_t)(2 * m) * nx + n * NT] = S.x * inv2;
+        Ck[(size_t)(2 * m + 1) * nx + n * NT] = S.y * inv2;
+      }
 }
 
-constexpr int BA_TZ = 64, BA_TX = 64, BA_KM = 8;  // apply tile: 64 z x 64 columns, 8 modes staged at a time
-constexpr int BA_THREADS = 256;                     // 4 x 4 outputs per thread
-
-// v[z][x] -= sum over the band's modes in order of (A_m cos_m(z) + B_m sin_m(z))
-__global__ void __launch_bounds__(BA_THREADS, 2)
-    band_apply_kernel(const __grid_constant__ ArrayList arrs, const double* __restrict__ W, int ldw, int J,
+// v[z][x] -= sum over the band's modes in order of (A_m cos_m(z) + B_m sin_m(z)),
+// 32 rows and 128 columns per CTA, 16 x 2 of them in a thread's registers: a
+// twiddle pair then serves eight FP64 instructions.
+constexpr int BA_NT = 128, BA_RZ = 16, BA_NC = 2;
+__global__ void __launch_bounds__(BA_NT)
+    band_apply_kernel(const __grid_constant__ ArrayList arrs, const double* __restrict__ W, int ldw, int M,
                       const double* __restrict__ C, int nx, int nz) {
-  __shared__ __align__(16) double sW[2][2 * BA_KM][BA_TZ + 1];  // [buffer][j][z]
-  __shared__ __align__(16) double sC[2][2 * BA_KM][BA_TX + 1];  // [buffer][j][x]
-  const int z0 = blockIdx.x * BA_TZ, x0 = blockIdx.y * BA_TX, k = blockIdx.z;
-  double* G = arrs.p[k];
-  const double* Ck = C + (size_t)k * J * nx;
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;  // ty -> z, tx -> x
-  double delta[4][4];
+  __shared__ __align__(16) double2 tw[2][BD_CH * BA_BM];
+  const int zh = (threadIdx.x >> 6) * BA_RZ;
+  const int z0 = blockIdx.x * BD_CH, x0 = blockIdx.y * BD_TX + (threadIdx.x & 63), k = blockIdx.z;
+  const double* c = C + (size_t)k * 2 * M * nx;
+  int xc[BA_NC];  // the columns whose coefficients are read
+  // Coefficients are read two modes ahead: they come from L2, and a mode takes
+  // a warp about as long as that.
+  double d[BA_NC][BA_RZ], nxt[2][2][BA_NC];
+  auto read = [&](int m) {
 #pragma unroll
-  for (int a = 0; a < 4; ++a)
+    for (int u = 0; u < 2; ++u) {
+      const double* r = c + (size_t)2 * min(m + u, M - 1) * nx;
 #pragma unroll
-    for (int b = 0; b < 4; ++b) delta[a][b] = 0.0;
-  auto stage = [&](int buf, int jb) {  // 8 modes (16 j) of W and of the coefficients, asynchronously
-    for (int i = threadIdx.x; i < 2 * BA_KM * BA_TZ; i += BA_THREADS) {
-      const int jj = i / BA_TZ, c = i - jj * BA_TZ;
-      const int j = jb + jj;
-      if (j < J && z0 + c < nz) cp_async8(&sW[buf][jj][c], W + (size_t)(z0 + c) * ldw + j);
-      else sW[buf][jj][c] = 0.0;
-      if (j < J && x0 + c < nx) cp_async8(&sC[buf][jj][c], Ck + (size_t)j * nx + x0 + c);
-      else sC[buf][jj][c] = 0.0;
+      for (int n = 0; n < BA_NC; ++n) {
+        nxt[u][0][n] = r[xc[n]];
+        nxt[u][1][n] = r[nx + xc[n]];
+      }
     }
-    cp_async_commit();
   };
-  const int nblk = (J + 2 * BA_KM - 1) / (2 * BA_KM);
-  stage(0, 0);
-  for (int blk = 0; blk < nblk; ++blk) {
-    const int buf = blk & 1, jb = blk * 2 * BA_KM;
-    if (blk + 1 < nblk) stage(buf ^ 1, jb + 2 * BA_KM);
-    else cp_async_commit();
-    cp_async_wait<1>();
-    __syncthreads();
-    const int mend = min(BA_KM, (J - jb) / 2);
-    for (int mm = 0; mm < mend; ++mm) {
-      double wc[4], ws[4], ca[4], cb[4];
+  stage_twiddles<BA_NT>(tw[0], W, ldw, z0, 0, BA_BM, nz, M);
 #pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        wc[a] = sW[buf][2 * mm][ty + 16 * a];
-        ws[a] = sW[buf][2 * mm + 1][ty + 16 * a];
-      }
+  for (int n = 0; n < BA_NC; ++n) {
+    xc[n] = min(x0 + n * 64, nx - 1);
 #pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        ca[b] = sC[buf][2 * mm][tx + 16 * b];
-        cb[b] = sC[buf][2 * mm + 1][tx + 16 * b];
-      }
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          const double t = ca[b] * wc[a] + cb[b] * ws[a];  // YM_Physics.cu:433 A_m cz + B_m sz
-          delta[a][b] = delta[a][b] + t;
-        }
-    }
-    __syncthreads();
+    for (int i = 0; i < BA_RZ; ++i) d[n][i] = 0.0;
   }
+  read(0);
+  const int nblk = (M + BA_BM - 1) / BA_BM;
+  for (int b = 0; b < nblk; ++b) {
+    cp_async_wait<0>();
+    __syncthreads();
+    if (b + 1 < nblk) stage_twiddles<BA_NT>(tw[(b + 1) & 1], W, ldw, z0, (b + 1) * BA_BM, BA_BM, nz, M);
+    const double2* t = tw[b & 1] + zh * BA_BM;
+    const int nm = min(BA_BM, M - b * BA_BM);
+    for (int m = 0; m < nm; m += 2) {
+      double cur[2][2][BA_NC];
 #pragma unroll
-  for (int a = 0; a < 4; ++a)
+      for (int u = 0; u < 2; ++u)
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const int z = z0 + ty + 16 * a, x = x0 + tx + 16 * b;
-      if (z < nz && x < nx) {
-        const size_t gi = idx2(x, z, nx);
-        G[gi] = G[gi] - delta[a][b];
+        for (int n = 0; n < BA_NC; ++n) {
+          cur[u][0][n] = nxt[u][0][n];
+          cur[u][1][n] = nxt[u][1][n];
+        }
+      read(b * BA_BM + m + 2);
+#pragma unroll
+      for (int u = 0; u < 2; ++u, ++t) {
+        if (m + u >= nm) break;
+#pragma unroll
+        for (int i = 0; i < BA_RZ; ++i) {
+          const double2 w = t[i * BA_BM];
+#pragma unroll
+          for (int n = 0; n < BA_NC; ++n) d[n][i] = d[n][i] + (cur[u][0][n] * w.x + cur[u][1][n] * w.y);  // YM_Physics.cu:433
+        }
       }
     }
+  }
+  double* g = arrs.p[k] + x0;
+#pragma unroll
+  for (int n = 0; n < BA_NC; ++n)
+    if (x0 + n * 64 < nx)
+#pragma unroll
+      for (int i = 0; i < BA_RZ; ++i)
+        if (z0 + zh + i < nz) g[(size_t)(z0 + zh + i) * nx + n * 64] -= d[n][i];
 }
+
+size_t band_coef_smem(int bm) { return sizeof(double2) * (size_t)bm * (2 * BD_CH + BD_TX); }
 
 cudaError_t launch_band(const ArrayList& arrs, int narr, const double* W, int ldw, int J, double* C, int nx, int nz,
                         double inv2, cudaStream_t s) {
-  dim3 g1((J + BC_TJ - 1) / BC_TJ, (nx + BC_TX - 1) / BC_TX, narr);
-  band_coef_kernel<<<g1, BC_THREADS, 0, s>>>(arrs, W, ldw, J, C, nx, nz, inv2);
+  const int M = J / 2, nxb = (nx + BD_TX - 1) / BD_TX;
+  // modes per coefficient CTA: as many as leave every SM some CTAs
+  int bm = BC_BM;
+  while (bm > 4 && (long long)((M + bm - 1) / bm) * nxb * narr < 148 * 4) bm /= 2;
+  bm = std::min(bm, M);
+  band_coef_kernel<<<dim3((M + bm - 1) / bm, nxb, narr), BC_NT, band_coef_smem(bm), s>>>(arrs, W, ldw, M, bm, C, nx, nz, inv2);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  dim3 g2((nz + BA_TZ - 1) / BA_TZ, (nx + BA_TX - 1) / BA_TX, narr);
-  band_apply_kernel<<<g2, BA_THREADS, 0, s>>>(arrs, W, ldw, J, C, nx, nz);
+  band_apply_kernel<<<dim3((nz + BD_CH - 1) / BD_CH, nxb, narr), BA_NT, 0, s>>>(arrs, W, ldw, M, C, nx, nz);
   return cudaGetLastError();
 }
 

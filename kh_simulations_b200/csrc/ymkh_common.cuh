@@ -156,6 +156,10 @@ __device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
   unsigned s = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
 }
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+  unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
@@ -170,6 +174,12 @@ namespace ymkh {
 struct ArrayList {
   double* p[24];
 };
+
+// Reversal of a 4-bit index: the order in which the band filter visits the
+// sixteen first-level nodes of the reference's warp tree (ymkh_column.cu).
+__host__ __device__ constexpr int bitrev4(int k) {
+  return ((k & 1) << 3) | ((k & 2) << 1) | ((k & 4) >> 1) | ((k & 8) >> 3);
+}
 
 // Arguments of the initial-state kernel (ymgpu2d/YM_Init.cu:32-40).
 struct InitArgs {
