@@ -59,7 +59,7 @@ struct NvtxRange {
     if (e_ != cudaSuccess) return set_err(YMKH_ECUDA, "%s: %s", what, cudaGetErrorString(e_)); \
   } while (0)
 
-constexpr int MAX_BANDS = 2 + YMKH_MAX_EXTRA_BANDS;
+constexpr int MAX_BANDS = kMaxBands;
 
 }  // namespace
 
@@ -90,14 +90,23 @@ struct ymkh_ctx {
   int sms = 148;
   bool aligned16 = false;   // every bound array 16-byte aligned: TMA bulk row copies allowed
   unsigned* derr = nullptr; // device error word of the bounded in-kernel waits
-  RunDesc* ddesc = nullptr; // device run descriptors for start buffer 0 and 1
-  RunDesc hdesc[2]{};       // their host copy, uploaded in stream order by the next step call
-  TensorMap* dmaps = nullptr; // device tensor maps: kFctMaps of buffer 0, then of buffer 1
-  TensorMap hmaps[2 * kFctMaps]{};  // their host copy, uploaded with hdesc
-  bool boxed = false;         // hmaps encoded: evenly spaced, 16-byte aligned arrays, nx even
+  // Tables of the kernels, uploaded in stream order by the next step call.
+  struct Tables {
+    TensorMap maps[2 * kFctMaps];  // kFctMaps of buffer 0, then of buffer 1
+    RunDesc desc[2];               // run descriptors for start buffer 0 and 1
+    ColDesc col[2];                // column stages writing buffer 0 and buffer 1
+  };
+  Tables host{};              // host copy
+  Tables* dev = nullptr;      // device copy
+  bool boxed = false;         // the maps encoded: evenly spaced, 16-byte aligned arrays, nx even
+  bool col_ok = false;        // the column stages can run as one kernel (ymkh_colfused.cu)
+  bool col_fused = false;     // and do, in a lone run
+  int col_items = 0;
+  size_t col_smem = 0;
+  unsigned version = 0;       // of the descriptors: a batch rebuilds its tables when a member's changed
   int fct_items = 0, mx_items = 0, fx_items = 0, fz_items = 0;
   bool desc_ok = false;
-  bool desc_pending = false; // hdesc not yet uploaded to ddesc
+  bool desc_pending = false; // host tables not yet uploaded
   int fct_mode = YMKH_FCT_FUSED;  // YMKH_FCT_FUSED or YMKH_FCT_SPLIT
   double* xscratch = nullptr;     // 12 x-swept fluid arrays of the split form
   int fz_seg = 128;
@@ -292,7 +301,7 @@ RunDesc make_desc(const ymkh_ctx* c, int start, int tb, int fct_item0, int mx_it
   d.fct_bulk = (c->aligned16 && fct_bulk_ok(c->sp, tb)) ? kAlignedRowLoad : (int)LOAD_ELEM;
   if (tb == 128 && d.fct_bulk != LOAD_ELEM && c->boxed) {
     d.fct_bulk = LOAD_BOX;
-    d.maps = c->dmaps + kFctMaps * start;
+    d.maps = c->dev->maps + kFctMaps * start;
   }
   d.mx_nstrips = maxwell_nstrips(c->nx);
   d.mx_seg = c->mx_seg;
@@ -354,51 +363,6 @@ bool encode_box(TensorMap* out, const State& s, int nx, int nz, int arrays, int 
                 CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Device descriptors of this run for both start buffers (single-run tables).
-int upload_desc(ymkh_ctx* c) {
-  c->desc_ok = false;
-  if (!c->bound) return 0;
-  if (!c->ddesc) CK(cudaMalloc(&c->ddesc, 2 * sizeof(RunDesc)), "cudaMalloc run descriptors");
-  { int rc = ensure_xscratch(c); if (rc) return rc; }
-  c->boxed = c->aligned16 && c->nx >= kFctBoxWidth;
-  constexpr int arrays[kFctMaps] = {12, 9, 1, 12, 9}, width[kFctMaps] = {kFctBoxWidth, kFctBoxWidth, kFctBoxWidth, 4, 4};
-  for (int k = 0; k < 2 * kFctMaps && c->boxed; ++k)
-    c->boxed = encode_box(&c->hmaps[k], c->buf[k / kFctMaps], c->nx, c->nz, arrays[k % kFctMaps], width[k % kFctMaps]);
-  if (c->boxed && !c->dmaps) CK(cudaMalloc(&c->dmaps, sizeof c->hmaps), "cudaMalloc tensor maps");
-  RunDesc* h = c->hdesc;
-  h[0] = make_desc(c, 0, c->fct_tx, 0, 0);
-  h[1] = make_desc(c, 1, c->fct_tx, 0, 0);
-  for (int i = 0; i < 2; ++i) h[i].fx_item0 = h[i].fz_item0 = 0;
-  c->fct_items = items_fct(h[0], c->nz);
-  c->mx_items = items_mx(h[0], c->nz);
-  c->fx_items = items_fx(h[0], c->nz);
-  c->fz_items = items_fz(h[0], c->nz);
-  c->desc_pending = true;  // uploaded by the next step call, on its stream
-  c->desc_ok = true;
-  return 0;
-}
-
-// Table uploads are ordered on the stream of the step call that follows a
-// change, after the steps already queued there, so a table is never
-// rewritten under a kernel in flight on that stream.  Inside a stream
-// capture (where a pageable copy cannot be captured) the copy is synchronous.
-cudaError_t upload_table(void* dst, const void* src, size_t bytes, cudaStream_t s) {
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (s) cudaStreamIsCapturing(s, &cs);
-  if (cs != cudaStreamCaptureStatusNone) return cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
-  return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s);
-}
-
-int flush_desc(ymkh_ctx* c, cudaStream_t s) {
-  if (!c->desc_ok) { int rc = upload_desc(c); if (rc) return rc; }
-  if (c->desc_pending) {
-    CK(upload_table(c->ddesc, c->hdesc, sizeof c->hdesc, s), "upload run descriptors");
-    if (c->boxed) CK(upload_table(c->dmaps, c->hmaps, sizeof c->hmaps, s), "upload tensor maps");
-    c->desc_pending = false;
-  }
-  return 0;
-}
-
 // The list l without its first k arrays.
 ArrayList drop_front(const ArrayList& l, int k) {
   ArrayList r{};
@@ -422,6 +386,106 @@ ArrayList list12(const State& s) {
   return l;
 }
 
+// The fused column stages' table for the run writing buffer `to`.
+ColDesc make_col(const ymkh_ctx* c, int to) {
+  ColDesc d{};
+  const ArrayList l = list21(c->buf[to]);
+  for (int i = 0; i < 21; ++i) d.arr[i] = l.p[i];
+  const ymkh_params& p = c->prm;
+  d.nx = c->nx; d.nz = c->nz; d.nb = c->nb;
+  for (int b = 0; b < c->nb; ++b) { d.W[b] = c->W[b]; d.M[b] = c->J[b] / 2; }
+  d.ncb = (c->nx + 31) / 32;
+  d.sponge = p.xi_sponge > 0.0; d.cut = p.xi_cut > 0.0; d.kz0 = p.suppress_kz0 != 0; d.hyper = p.hyp_diff_coeff > 0.0;
+  d.k0 = (c->nb || d.kz0) ? 0 : 3;
+  d.dx = c->sp.dx; d.dt = c->sp.dt; d.epsilon = c->sp.epsilon; d.xi_sponge = c->sp.xi_sponge;
+  d.sigma_sponge = c->sp.sigma_sponge; d.xi_cut = c->sp.xi_cut; d.hyp_diff = c->sp.hyp_diff;
+  d.inv2 = (double)(2.0f / (float)c->nz);
+  return d;
+}
+
+// Arrays the fused column stages visit: all 21 with bands, else colours 2 and
+// 3 (and colour 1, to zero it, with suppress_kz0).
+int col_arrays(const ColDesc& d) { return d.nb ? 21 : (d.kz0 ? 15 : 12); }
+
+int band_modes(const ymkh_ctx* c) {  // of the widest band
+  int m = 0;
+  for (int b = 0; b < c->nb; ++b) m = std::max(m, c->J[b] / 2);
+  return m;
+}
+
+// Whether the column stages can run as one kernel (ymkh_colfused.cu).
+bool col_fused_ok(const ymkh_ctx* c) {
+  const ymkh_params& p = c->prm;
+  if (c->nz % 32 || c->nz > kColumnFusedMaxNz) return false;
+  if (c->nb && p.filter_engine != YMKH_FILTER_DFT) return false;
+  if (!c->nb && !p.suppress_kz0 && p.xi_sponge <= 0.0 && p.xi_cut <= 0.0 && p.hyp_diff_coeff <= 0.0) return false;
+  return column_fused_smem(c->nz, band_modes(c), p.suppress_kz0) <= kColumnFusedSmemMax;
+}
+
+// Whether a lone run takes that kernel: with two stages or more, or with band
+// filters alone up to 128 rows.  Step us, one kernel against separate ones:
+// all stages 64 x 768 54 / 72, 256 x 768 120 / 149, 512 x 1024 248 / 306;
+// z-mean and band 512 x 1024 664 / 686; band alone 64 x 192 35 / 43,
+// 96 x 512 56 / 59, but 256 x 512 169 / 161, 512 x 512 483 / 423 (its CTAs
+// have a column tile each and end unevenly); z-mean alone 256 x 256 55 / 54,
+// 512 x 1024 140 / 132.
+bool col_fused_alone(const ymkh_ctx* c) {
+  const ymkh_params& p = c->prm;
+  const int stages = (p.xi_sponge > 0.0 || p.xi_cut > 0.0) + (p.suppress_kz0 != 0) + (c->nb > 0) + (p.hyp_diff_coeff > 0.0);
+  return stages >= 2 || (c->nb && c->nz <= 128);
+}
+
+// Device descriptors of this run for both start buffers (single-run tables).
+int upload_desc(ymkh_ctx* c) {
+  c->desc_ok = false;
+  if (!c->bound) return 0;
+  if (!c->dev) CK(cudaMalloc(&c->dev, sizeof(ymkh_ctx::Tables)), "cudaMalloc run tables");
+  { int rc = ensure_xscratch(c); if (rc) return rc; }
+  c->boxed = c->aligned16 && c->nx >= kFctBoxWidth;
+  constexpr int arrays[kFctMaps] = {12, 9, 1, 12, 9}, width[kFctMaps] = {kFctBoxWidth, kFctBoxWidth, kFctBoxWidth, 4, 4};
+  for (int k = 0; k < 2 * kFctMaps && c->boxed; ++k)
+    c->boxed = encode_box(&c->host.maps[k], c->buf[k / kFctMaps], c->nx, c->nz, arrays[k % kFctMaps], width[k % kFctMaps]);
+  RunDesc* h = c->host.desc;
+  h[0] = make_desc(c, 0, c->fct_tx, 0, 0);
+  h[1] = make_desc(c, 1, c->fct_tx, 0, 0);
+  for (int i = 0; i < 2; ++i) h[i].fx_item0 = h[i].fz_item0 = 0;
+  c->fct_items = items_fct(h[0], c->nz);
+  c->mx_items = items_mx(h[0], c->nz);
+  c->fx_items = items_fx(h[0], c->nz);
+  c->fz_items = items_fz(h[0], c->nz);
+  c->col_ok = col_fused_ok(c);
+  c->col_fused = c->col_ok && col_fused_alone(c);
+  if (c->col_ok) {
+    for (int i = 0; i < 2; ++i) c->host.col[i] = make_col(c, i);
+    c->col_smem = column_fused_smem(c->nz, band_modes(c), c->prm.suppress_kz0);
+    c->col_items = c->host.col[0].ncb * col_arrays(c->host.col[0]);
+  }
+  ++c->version;
+  c->desc_pending = true;  // uploaded by the next step call, on its stream
+  c->desc_ok = true;
+  return 0;
+}
+
+// Table uploads are ordered on the stream of the step call that follows a
+// change, after the steps already queued there, so a table is never
+// rewritten under a kernel in flight on that stream.  Inside a stream
+// capture (where a pageable copy cannot be captured) the copy is synchronous.
+cudaError_t upload_table(void* dst, const void* src, size_t bytes, cudaStream_t s) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (s) cudaStreamIsCapturing(s, &cs);
+  if (cs != cudaStreamCaptureStatusNone) return cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+  return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s);
+}
+
+int flush_desc(ymkh_ctx* c, cudaStream_t s) {
+  if (!c->desc_ok) { int rc = upload_desc(c); if (rc) return rc; }
+  if (c->desc_pending) {
+    CK(upload_table(c->dev, &c->host, sizeof c->host, s), "upload run tables");
+    c->desc_pending = false;
+  }
+  return 0;
+}
+
 // One reference iteration from buffer c->cur into buffer 1 - c->cur.
 enum Stage { ST_FCT = 0, ST_MAXWELL, ST_POINTWISE, ST_ZMEAN, ST_BANDS, ST_HYPER, ST_ZERO, ST_COUNT };
 
@@ -430,8 +494,19 @@ void mark(ymkh_ctx* c, int stage, cudaStream_t s) {
 }
 
 // Stages after the fused FCT and Maxwell launches, on the run's new buffer.
-int post_stages(ymkh_ctx* c, const State& out, cudaStream_t s) {
+int post_stages(ymkh_ctx* c, cudaStream_t s) {
+  const State& out = c->buf[1 - c->cur];
   mark(c, ST_POINTWISE, s);
+  if (c->col_fused) {
+    mark(c, ST_ZMEAN, s);
+    mark(c, ST_BANDS, s);
+    CK(launch_column_fused(c->dev->col + (1 - c->cur), 1, c->col_items, c->nz, c->col_smem, s), "column stages");
+    g_launches++;
+    mark(c, ST_HYPER, s);
+    mark(c, ST_ZERO, s);
+    mark(c, ST_COUNT, s);
+    return 0;
+  }
   if (c->prm.xi_sponge > 0.0) { CK(launch_sponge_xicut(list12(out), c->sp, 0, s), "sponge"); g_launches++; }
   if (c->prm.xi_cut > 0.0) { CK(launch_sponge_xicut(list12(out), c->sp, 1, s), "xi_cut"); g_launches++; }
   // With suppress_kz0 the step ends by zeroing By1, Ex1 and Ez1, the first
@@ -471,10 +546,15 @@ int post_stages(ymkh_ctx* c, const State& out, cudaStream_t s) {
   return 0;
 }
 
+bool has_column_stages(const ymkh_ctx* c) {
+  const ymkh_params& p = c->prm;
+  return c->nb || p.suppress_kz0 || p.xi_sponge > 0.0 || p.xi_cut > 0.0 || p.hyp_diff_coeff > 0.0;
+}
+
 // One reference iteration from buffer c->cur into buffer 1 - c->cur.
 int step_once(ymkh_ctx* c, cudaStream_t s) {
   { int rc = flush_desc(c, s); if (rc) return rc; }
-  RunTable T{c->ddesc + c->cur, 1, c->fct_items, c->mx_items, c->derr, c->fx_items, c->fz_items, 1};
+  RunTable T{c->dev->desc + c->cur, 1, c->fct_items, c->mx_items, c->derr, c->fx_items, c->fz_items, 1};
   mark(c, ST_FCT, s);
   {
     NvtxRange r("ymkh fct");
@@ -492,7 +572,7 @@ int step_once(ymkh_ctx* c, cudaStream_t s) {
   }
   g_launches += 2;
   NvtxRange r("ymkh column stages");
-  int rc = post_stages(c, c->buf[1 - c->cur], s);
+  int rc = post_stages(c, s);
   if (rc) return rc;
   c->cur = 1 - c->cur;
   return 0;
@@ -577,6 +657,7 @@ int ymkh_create(const ymkh_grid* grid, const ymkh_params* params, ymkh_ctx** out
   CK_CREATE(prepare_fct(128), "FCT kernel attributes");
   CK_CREATE(prepare_maxwell(), "Maxwell kernel attributes");
   CK_CREATE(prepare_fct_split(), "split FCT kernel attributes");
+  CK_CREATE(prepare_column_fused(), "column kernel attributes");
   choose_launch_shape(c);
   CK_CREATE(prepare_column(c->nz), "column kernel attributes");
 #undef CK_CREATE
@@ -895,8 +976,7 @@ int ymkh_destroy(ymkh_ctx* c) {
   if (c->mweight) cudaFree(c->mweight);
   if (c->gpart) cudaFree(c->gpart);
   if (c->derr) cudaFree(c->derr);
-  if (c->ddesc) cudaFree(c->ddesc);
-  if (c->dmaps) cudaFree(c->dmaps);
+  if (c->dev) cudaFree(c->dev);
   if (c->xscratch) cudaFree(c->xscratch);
   delete c;
   return 0;
@@ -927,6 +1007,12 @@ struct ymkh_batch {
   std::vector<ymkh_ctx*> runs;
   RunDesc* ddesc = nullptr;  // [2][cap]: tables for the members' current / next buffers
   int cap = 0;
+  // members whose column stages run fused, grouped by NZ (one launch a group)
+  struct ColGroup { int nz, first, n, items; size_t smem; };
+  ColDesc* dcol = nullptr;   // [2][cap]
+  std::vector<ColGroup> col;
+  std::vector<char> col_member;    // whether the member is in one of the groups
+  std::vector<unsigned> versions;  // of the members' descriptors when the tables were built
   int fct_items = 0, mx_items = 0, fx_items = 0, fz_items = 0;
   int tb = 128, fct_grid = 0, mx_grid = 0, fx_grid = 0, fz_grid = 0;
   int fct_mode = YMKH_FCT_FUSED;
@@ -955,9 +1041,15 @@ void batch_drop_graph(ymkh_batch* b) {
 int batch_build(ymkh_batch* b, cudaStream_t s) {
   const int n = (int)b->runs.size();
   if (n > b->cap) {
+    const int cap = std::max(n, 2 * b->cap);
     if (b->ddesc) cudaFree(b->ddesc);
-    b->cap = std::max(n, 2 * b->cap);
-    CK(cudaMalloc(&b->ddesc, 2 * (size_t)b->cap * sizeof(RunDesc)), "cudaMalloc batch descriptors");
+    if (b->dcol) cudaFree(b->dcol);
+    b->ddesc = nullptr;
+    b->dcol = nullptr;
+    b->cap = 0;
+    CK(cudaMalloc(&b->dcol, 2 * (size_t)cap * sizeof(ColDesc)), "cudaMalloc batch column tables");
+    CK(cudaMalloc(&b->ddesc, 2 * (size_t)cap * sizeof(RunDesc)), "cudaMalloc batch descriptors");
+    b->cap = cap;
   }
   std::vector<RunDesc> h(2 * (size_t)std::max(n, 1));
   std::vector<MxGrid> mg;
@@ -1002,6 +1094,39 @@ int batch_build(ymkh_batch* b, cudaStream_t s) {
     CK(upload_table(b->ddesc, h.data(), (size_t)n * sizeof(RunDesc), s), "upload batch table");
     CK(upload_table(b->ddesc + b->cap, h.data() + n, (size_t)n * sizeof(RunDesc), s), "upload batch table");
   }
+  // fused column stages: members sorted by NZ, one table range and launch per NZ
+  b->col.clear();
+  b->versions.clear();
+  std::vector<int> order;
+  int n_ok = 0;
+  for (int i = 0; i < n; ++i) {
+    b->versions.push_back(b->runs[i]->version);
+    n_ok += b->runs[i]->col_ok;
+  }
+  // one launch per NZ for all members that can, once they are several: what a
+  // member loses to its own kernels is less than its launches
+  b->col_member.assign(n, 0);
+  for (int i = 0; i < n; ++i)
+    if (n_ok >= 4 ? b->runs[i]->col_ok : b->runs[i]->col_fused) {
+      b->col_member[i] = 1;
+      order.push_back(i);
+    }
+  std::stable_sort(order.begin(), order.end(), [&](int i, int j) { return b->runs[i]->nz < b->runs[j]->nz; });
+  std::vector<ColDesc> hc[2];
+  for (int i : order) {
+    ymkh_ctx* c = b->runs[i];
+    if (b->col.empty() || b->col.back().nz != c->nz) b->col.push_back({c->nz, (int)hc[0].size(), 0, 0, 0});
+    ymkh_batch::ColGroup& g = b->col.back();
+    for (int p = 0; p < 2; ++p) {
+      hc[p].push_back(c->host.col[p ? c->cur : 1 - c->cur]);
+      hc[p].back().item0 = g.items;
+    }
+    g.n++;
+    g.items += c->col_items;
+    g.smem = std::max(g.smem, c->col_smem);
+  }
+  for (int p = 0; p < 2 && !order.empty(); ++p)
+    CK(upload_table(b->dcol + (size_t)p * b->cap, hc[p].data(), hc[p].size() * sizeof(ColDesc), s), "upload batch column table");
   b->parity = 0;
   b->dirty = false;
   batch_drop_graph(b);
@@ -1018,15 +1143,31 @@ int batch_step_once(ymkh_batch* b, cudaStream_t s) {
     CK(launch_fct_table(T, b->tb, b->fct_grid, s), "fct_fused_kernel (batch)");
   CK(launch_maxwell_table(T, b->mx_grid, s), "maxwell_fused_kernel (batch)");
   g_launches += 2;
-  const int na = b->aux[0] ? std::min(n, (int)ymkh_batch::kAux) : 1;
+  // column stages: one launch per NZ of the fused ones, the others per member;
+  // all independent of each other, spread over the auxiliary streams
+  auto separate = [&](int i) { return !b->col_member[i] && has_column_stages(b->runs[i]); };
+  int nsep = 0;
+  for (int i = 0; i < n; ++i) nsep += separate(i);
+  const int jobs = (int)b->col.size() + nsep;
+  const int na = b->aux[0] ? std::min(jobs, (int)ymkh_batch::kAux) : 1;
   if (na > 1) {
     CK(cudaEventRecord(b->fork_ev, s), "batch fork");
     for (int i = 0; i < na; ++i) CK(cudaStreamWaitEvent(b->aux[i], b->fork_ev, 0), "batch fork");
   }
-  for (int j = 0; j < n; ++j) {
-    ymkh_ctx* c = b->runs[j];
-    int rc = post_stages(c, c->buf[1 - c->cur], na > 1 ? b->aux[j % na] : s);
-    if (rc) return rc;
+  int job = 0;
+  for (const ymkh_batch::ColGroup& g : b->col) {
+    CK(launch_column_fused(b->dcol + (size_t)b->parity * b->cap + g.first, g.n, g.items, g.nz, g.smem,
+                           na > 1 ? b->aux[job % na] : s), "column stages (batch)");
+    g_launches++;
+    ++job;
+  }
+  for (int i = 0; i < n; ++i) {
+    ymkh_ctx* c = b->runs[i];
+    if (separate(i)) {
+      int rc = post_stages(c, na > 1 ? b->aux[job % na] : s);
+      if (rc) return rc;
+      ++job;
+    }
     c->cur = 1 - c->cur;
   }
   if (na > 1) {
@@ -1104,6 +1245,7 @@ int ymkh_batch_step(ymkh_batch* b, int nsteps, void* stream) {
   if (nsteps < 0) return set_err(YMKH_EINVAL, "negative step count");
   NvtxRange range("ymkh_batch_step");
   cudaStream_t s = (cudaStream_t)stream;
+  for (size_t i = 0; i < b->versions.size() && !b->dirty; ++i) b->dirty = b->versions[i] != b->runs[i]->version;
   if (b->dirty) { int rc = batch_build(b, s); if (rc) return rc; }
   int done = 0;
   const bool graphs = s != nullptr && b->graph_steps >= 2 && !b->runs.empty();
@@ -1184,6 +1326,7 @@ int ymkh_batch_destroy(ymkh_batch* b) {
   if (!b) return 0;
   batch_drop_graph(b);
   if (b->ddesc) cudaFree(b->ddesc);
+  if (b->dcol) cudaFree(b->dcol);
   if (b->derr) cudaFree(b->derr);
   for (int i = 0; i < ymkh_batch::kAux; ++i) {
     if (b->aux[i]) cudaStreamDestroy(b->aux[i]);

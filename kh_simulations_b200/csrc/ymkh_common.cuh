@@ -181,6 +181,24 @@ __host__ __device__ constexpr int bitrev4(int k) {
   return ((k & 1) << 3) | ((k & 2) << 1) | ((k & 4) >> 1) | ((k & 8) >> 3);
 }
 
+constexpr int kMaxBands = 2 + YMKH_MAX_EXTRA_BANDS;
+
+// One run's column stages as the fused kernel sees them (ymkh_colfused.cu).
+struct ColDesc {
+  double* arr[21];          // the filtered arrays of the new state
+  const double* W[kMaxBands];
+  int M[kMaxBands];         // modes per band
+  int nx, nz, nb;
+  int item0, ncb, k0;       // first CTA, 32-column blocks, first array
+  int sponge, cut, kz0, hyper;
+  double dx, dt, epsilon, xi_sponge, sigma_sponge, xi_cut, hyp_diff, inv2;
+};
+constexpr int kColumnFusedMaxNz = 512;
+constexpr size_t kColumnFusedSmemMax = 200 * 1024;
+size_t column_fused_smem(int nz, int max_modes, int kz0);
+cudaError_t prepare_column_fused();
+cudaError_t launch_column_fused(const ColDesc* dev, int n, int items, int nz, size_t smem, cudaStream_t s);
+
 // Arguments of the initial-state kernel (ymgpu2d/YM_Init.cu:32-40).
 struct InitArgs {
   int nx, nz;
