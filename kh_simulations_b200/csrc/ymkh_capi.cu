@@ -21,6 +21,7 @@
 #include <cstring>
 #include <cstdarg>
 #include <atomic>
+#include <mutex>
 #include <vector>
 #include <algorithm>
 #include "ymkh_common.cuh"
@@ -61,6 +62,62 @@ struct NvtxRange {
 
 constexpr int MAX_BANDS = kMaxBands;
 
+// Pages of pinned host memory that the diagnostics' last kernels write their
+// results to, one slot of 32 doubles per context: reading a result back is
+// then the stream's synchronisation alone, where a copy to the caller's
+// pageable memory is staged and synchronised by itself.  Slots come from
+// 64 KiB slabs shared by all contexts of the process (any device, any
+// thread); a slab whose slots are all given back is freed, but for one kept.
+class HostSlots {
+ public:
+  static constexpr int kDoubles = 32, kPerSlab = 256;
+  double* take() {
+    std::lock_guard<std::mutex> lock(mu_);
+    for (Slab& s : slabs_)
+      if (s.used < kPerSlab)
+        for (int i = 0; i < kPerSlab; ++i)
+          if (!s.taken[i]) return give_out(s, i);
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, sizeof(double) * kDoubles * kPerSlab, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess)
+      return nullptr;
+    slabs_.push_back(Slab{static_cast<double*>(p), 0, std::vector<char>(kPerSlab, 0)});
+    return give_out(slabs_.back(), 0);
+  }
+  void give_back(double* slot) {
+    std::lock_guard<std::mutex> lock(mu_);
+    int empty = 0;
+    for (size_t k = 0; k < slabs_.size(); ++k) {
+      Slab& s = slabs_[k];
+      if (slot >= s.base && slot < s.base + kDoubles * kPerSlab) {
+        s.taken[(slot - s.base) / kDoubles] = 0;
+        --s.used;
+      }
+      if (!s.used && empty++) {
+        cudaFreeHost(s.base);
+        slabs_.erase(slabs_.begin() + k--);
+      }
+    }
+  }
+
+ private:
+  struct Slab {
+    double* base;
+    int used;
+    std::vector<char> taken;
+  };
+  double* give_out(Slab& s, int i) {
+    s.taken[i] = 1;
+    ++s.used;
+    return s.base + (size_t)i * kDoubles;
+  }
+  std::mutex mu_;
+  std::vector<Slab> slabs_;
+};
+HostSlots& host_slots() {
+  static HostSlots* p = new HostSlots();  // not destroyed: contexts may outlive static objects
+  return *p;
+}
+
 }  // namespace
 
 struct ymkh_ctx {
@@ -80,10 +137,10 @@ struct ymkh_ctx {
   Tf32BandImages tfb[MAX_BANDS]{};  // TF32 engine: twiddle tile images per band
   Tf32Scratch tfs{};                // TF32 engine: G and C^T tile images
   double* epart = nullptr;   // energy partials
-  double* edev = nullptr;    // [0] energy, [1..2] mode amplitudes
-  double* mcol = nullptr;    // mode amplitude per-column buffer
+  double* hres = nullptr;    // results of the diagnostics: a slot of pinned host memory (on first use)
+  double* mcol = nullptr;    // mode amplitude partial sums (allocated on first use)
   double* mweight = nullptr; // x weights of ymkh_circ_amp (NX doubles, allocated on first use)
-  double* gpart = nullptr;   // Gauss residual partials and results (allocated on first use)
+  double* gpart = nullptr;   // Gauss residual partials (allocated on first use)
   SnapshotQueue* snaps = nullptr;  // snapshot writers (created on first use)
   int fct_tx = 64, fct_seg = 16, fct_grid = 296;  // FCT threads per beam, segment rows, persistent CTAs
   int mx_seg = 16, mx_grid = 148;                   // Maxwell segment rows, persistent CTAs
@@ -663,8 +720,6 @@ int ymkh_create(const ymkh_grid* grid, const ymkh_params* params, ymkh_ctx** out
 #undef CK_CREATE
   const int np = energy_nparts(c->N);
   if (cudaMalloc(&c->epart, (size_t)2 * np * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&c->edev, 4 * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&c->mcol, (size_t)2 * c->nx * sizeof(double)) != cudaSuccess ||
       cudaMalloc(&c->derr, sizeof(unsigned)) != cudaSuccess || cudaMemset(c->derr, 0, sizeof(unsigned)) != cudaSuccess) {
     ymkh_destroy(c);
     return set_err(YMKH_ENOMEM, "cudaMalloc diagnostics");
@@ -888,17 +943,28 @@ int ymkh_stage_times(ymkh_ctx* c, int nsteps, void* stream, float* out_ms, int n
 int ymkh_energy_async(ymkh_ctx* c, double* dev_out, void* stream) {
   if (!c || !dev_out) return set_err(YMKH_EINVAL, "null argument");
   if (!c->bound) return set_err(YMKH_ESTATE, "state not bound");
-  CK(launch_energy(c->buf[c->cur], c->N, c->epart, dev_out, (cudaStream_t)stream), "energy kernels");
+  CK(launch_energy(c->buf[c->cur], c->N, c->epart, dev_out, nullptr, (cudaStream_t)stream), "energy kernels");
   g_launches += 2;
+  return 0;
+}
+
+// Slot of the diagnostics' results.
+static int host_result(ymkh_ctx* c) {
+  if (!c->hres && !(c->hres = host_slots().take())) return set_err(YMKH_ENOMEM, "cudaHostAlloc diagnostics page");
   return 0;
 }
 
 int ymkh_energy(ymkh_ctx* c, double* host_out, void* stream) {
   if (!host_out) return set_err(YMKH_EINVAL, "null argument");
-  int rc = ymkh_energy_async(c, c ? c->edev : nullptr, stream);
-  if (rc) return rc;
-  CK(cudaMemcpyAsync(host_out, c->edev, sizeof(double), cudaMemcpyDeviceToHost, (cudaStream_t)stream), "energy D2H");
-  return ymkh_check(c, stream);
+  if (!c) return set_err(YMKH_EINVAL, "null argument");
+  if (!c->bound) return set_err(YMKH_ESTATE, "state not bound");
+  { int rc = host_result(c); if (rc) return rc; }
+  cudaStream_t s = (cudaStream_t)stream;
+  CK(launch_energy(c->buf[c->cur], c->N, c->epart, c->hres, c->derr, s), "energy kernels");
+  g_launches += 2;
+  CK(cudaStreamSynchronize(s), "energy sync");
+  *host_out = c->hres[0];
+  return c->hres[1] != 0.0 ? ymkh_check(c, stream) : 0;  // reports and clears the error word
 }
 
 int ymkh_mode_amp(ymkh_ctx* c, int k, double* host_out2, void* stream) {
@@ -912,6 +978,9 @@ int ymkh_circ_amp(ymkh_ctx* c, int pair, int k, const double* host_weight, doubl
   if (pair < 0 || pair > 3) return set_err(YMKH_EINVAL, "pair %d not in 0..3", pair);
   cudaStream_t s = (cudaStream_t)stream;
   const State& st = c->buf[c->cur];
+  { int rc = host_result(c); if (rc) return rc; }
+  if (!c->mcol && cudaMalloc(&c->mcol, mode_amp_scratch(c->nx, c->nz) * sizeof(double)) != cudaSuccess)
+    return set_err(YMKH_ENOMEM, "cudaMalloc mode amplitude scratch");
   const double* w = nullptr;
   if (host_weight) {
     if (!c->mweight && cudaMalloc(&c->mweight, (size_t)c->nx * sizeof(double)) != cudaSuccess)
@@ -920,11 +989,12 @@ int ymkh_circ_amp(ymkh_ctx* c, int pair, int k, const double* host_weight, doubl
        "mode weights H2D");
     w = c->mweight;
   }
-  CK(launch_mode_amp(st.f[re_of[pair]], st.f[re_of[pair] + 1], c->nx, c->nz, k, c->mcol, w, c->edev + 1, s),
+  CK(launch_mode_amp(st.f[re_of[pair]], st.f[re_of[pair] + 1], c->nx, c->nz, k, c->mcol, w, c->hres, s),
      "mode amplitude kernels");
   g_launches += 2;
-  CK(cudaMemcpyAsync(host_out2, c->edev + 1, 2 * sizeof(double), cudaMemcpyDeviceToHost, s), "mode amp D2H");
   CK(cudaStreamSynchronize(s), "mode amp sync");
+  host_out2[0] = c->hres[0];
+  host_out2[1] = c->hres[1];
   return 0;
 }
 
@@ -932,16 +1002,16 @@ int ymkh_gauss(ymkh_ctx* c, double* host_out, void* stream) {
   if (!c || !host_out) return set_err(YMKH_EINVAL, "null argument");
   if (!c->bound) return set_err(YMKH_ESTATE, "state not bound");
   const int np = gauss_nparts(c->N);
-  const size_t n = (size_t)np * YMKH_GAUSS_NOUT * 2 + YMKH_GAUSS_NOUT;
+  const size_t n = (size_t)np * YMKH_GAUSS_NOUT * 2;
+  { int rc = host_result(c); if (rc) return rc; }
   if (!c->gpart && cudaMalloc(&c->gpart, n * sizeof(double)) != cudaSuccess)
     return set_err(YMKH_ENOMEM, "cudaMalloc Gauss partials");
   cudaStream_t s = (cudaStream_t)stream;
-  double* dout = c->gpart + (size_t)np * YMKH_GAUSS_NOUT * 2;
-  CK(launch_gauss(c->buf[c->cur], c->nx, c->nz, c->prm.dx, c->prm.dz, c->prm.alpha_YM, c->gpart, dout, s),
+  CK(launch_gauss(c->buf[c->cur], c->nx, c->nz, c->prm.dx, c->prm.dz, c->prm.alpha_YM, c->gpart, c->hres, s),
      "Gauss residual kernels");
   g_launches += 2;
-  CK(cudaMemcpyAsync(host_out, dout, YMKH_GAUSS_NOUT * sizeof(double), cudaMemcpyDeviceToHost, s), "Gauss D2H");
   CK(cudaStreamSynchronize(s), "Gauss sync");
+  for (int i = 0; i < YMKH_GAUSS_NOUT; ++i) host_out[i] = c->hres[i];
   return 0;
 }
 
@@ -971,7 +1041,7 @@ int ymkh_destroy(ymkh_ctx* c) {
   free_bands(c);
   if (c->own) cudaFree(c->own);
   if (c->epart) cudaFree(c->epart);
-  if (c->edev) cudaFree(c->edev);
+  if (c->hres) host_slots().give_back(c->hres);
   if (c->mcol) cudaFree(c->mcol);
   if (c->mweight) cudaFree(c->mweight);
   if (c->gpart) cudaFree(c->gpart);

@@ -516,147 +516,4 @@ cudaError_t launch_band(const ArrayList& arrs, int narr, const double* W, int ld
   return cudaGetLastError();
 }
 
-// ---------------------------------------------------------------- energy
-// Per-cell energy of YM_Energy.cu:3-21, summed with Neumaier compensation in
-// a fixed order: each CTA reduces a contiguous block of cells, a second
-// single-CTA pass reduces the CTA partials in index order.
-constexpr int EN_THREADS = 256;
-constexpr int EN_PER_THREAD = 16;
-
-__global__ void __launch_bounds__(EN_THREADS)
-    energy_partial_kernel(const __grid_constant__ State st, size_t N, double* __restrict__ part) {
-  const size_t base = (size_t)blockIdx.x * EN_THREADS * EN_PER_THREAD;
-  double s = 0.0, c = 0.0;
-  for (int k = 0; k < EN_PER_THREAD; ++k) {
-    const size_t i = base + (size_t)k * EN_THREADS + threadIdx.x;
-    if (i >= N) break;
-    const double nA = fmax(st.a[FN][i], 1e-10);
-    const double nB = fmax(st.b[FN][i], 1e-10);
-    const double pxA = st.a[FPX][i], pzA = st.a[FPZ][i], pxB = st.b[FPX][i], pzB = st.b[FPZ][i];
-    const double keA = 0.5 * (pxA * pxA + pzA * pzA) / nA;
-    const double keB = 0.5 * (pxB * pxB + pzB * pzB) / nB;
-    double em2 = 0.0;
-    em2 = st.f[EX1][i] * st.f[EX1][i];
-    em2 = em2 + st.f[EX2][i] * st.f[EX2][i];
-    em2 = em2 + st.f[EX3][i] * st.f[EX3][i];
-    em2 = em2 + st.f[EZ1][i] * st.f[EZ1][i];
-    em2 = em2 + st.f[EZ2][i] * st.f[EZ2][i];
-    em2 = em2 + st.f[EZ3][i] * st.f[EZ3][i];
-    em2 = em2 + st.f[BY1][i] * st.f[BY1][i];
-    em2 = em2 + st.f[BY2][i] * st.f[BY2][i];
-    em2 = em2 + st.f[BY3][i] * st.f[BY3][i];
-    const double e = keA + keB + 0.5 * em2;
-    neumaier_add(s, c, e);
-  }
-  __shared__ double ss[EN_THREADS], sc[EN_THREADS];
-  ss[threadIdx.x] = s;
-  sc[threadIdx.x] = c;
-  __syncthreads();
-  for (int w = EN_THREADS / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) {
-      double a = ss[threadIdx.x], ca = sc[threadIdx.x] + sc[threadIdx.x + w];
-      neumaier_add(a, ca, ss[threadIdx.x + w]);
-      ss[threadIdx.x] = a;
-      sc[threadIdx.x] = ca;
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    part[2 * blockIdx.x] = ss[0];
-    part[2 * blockIdx.x + 1] = sc[0];
-  }
-}
-
-__global__ void energy_final_kernel(const double* __restrict__ part, int nparts, double* out) {
-  __shared__ double ss[256], sc[256];
-  double s = 0.0, c = 0.0;
-  // thread t reduces a contiguous slice of the partials, in order
-  const int per = (nparts + 255) / 256;
-  for (int k = 0; k < per; ++k) {
-    const int i = threadIdx.x * per + k;
-    if (i >= nparts) break;
-    c += part[2 * i + 1];
-    neumaier_add(s, c, part[2 * i]);
-  }
-  ss[threadIdx.x] = s;
-  sc[threadIdx.x] = c;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double a = 0.0, ca = 0.0;
-    for (int t = 0; t < 256; ++t) {
-      ca += sc[t];
-      neumaier_add(a, ca, ss[t]);
-    }
-    *out = a + ca;
-  }
-}
-
-int energy_nparts(size_t N) { return (int)((N + EN_THREADS * EN_PER_THREAD - 1) / (EN_THREADS * EN_PER_THREAD)); }
-
-cudaError_t launch_energy(const State& st, size_t N, double* part, double* out, cudaStream_t s) {
-  const int np = energy_nparts(N);
-  energy_partial_kernel<<<np, EN_THREADS, 0, s>>>(st, N, part);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  energy_final_kernel<<<1, 256, 0, s>>>(part, np, out);
-  return cudaGetLastError();
-}
-
-// ------------------------------------------------------------ mode amplitude
-// Per column x, F = sum_z (re + i im) e^{-2 pi i k z/nz} and Fc for re - i im
-// (ymgpu2d/analysis/remote_timeseries.py:62-77 for re, im = Az2, Az3;
-// ymgpu2d/analysis/resolution_convergence.py:83-86 for By2, By3).
-__global__ void mode_amp_kernel(const double* __restrict__ re, const double* __restrict__ im, int nx, int nz,
-                                int k, double* __restrict__ colbuf) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= nx) return;
-  double fr = 0, fi = 0, cr = 0, ci = 0;
-  for (int z = 0; z < nz; ++z) {
-    double sn, cs;
-    sincospi(-2.0 * (double)k * (double)z / (double)nz, &sn, &cs);
-    const double a = re[idx2(x, z, nx)], b = im[idx2(x, z, nx)];
-    // (a + i b)(cs + i sn)
-    fr += a * cs - b * sn;
-    fi += a * sn + b * cs;
-    // (a - i b)(cs + i sn)
-    cr += a * cs + b * sn;
-    ci += a * sn - b * cs;
-  }
-  colbuf[2 * x] = hypot(fr, fi);
-  colbuf[2 * x + 1] = hypot(cr, ci);
-}
-
-// Without a weight: (mean_x |F| / nz, mean_x |Fc| / nz), remote_timeseries.py:72-74.
-// With one: (sum_x w[x] |F| / nz, sum_x w[x] |Fc| / nz), the shear-layer
-// weighted average of resolution_convergence.py:83-86.
-__global__ void mode_amp_final_kernel(const double* __restrict__ colbuf, const double* __restrict__ w, int nx, int nz,
-                                      double* out) {
-  if (threadIdx.x != 0) return;
-  double s0 = 0, s1 = 0;
-  if (w == nullptr) {
-    for (int x = 0; x < nx; ++x) {
-      s0 += colbuf[2 * x];
-      s1 += colbuf[2 * x + 1];
-    }
-    out[0] = s0 / nx / nz;
-    out[1] = s1 / nx / nz;
-  } else {
-    for (int x = 0; x < nx; ++x) {
-      s0 += w[x] * (colbuf[2 * x] / nz);
-      s1 += w[x] * (colbuf[2 * x + 1] / nz);
-    }
-    out[0] = s0;
-    out[1] = s1;
-  }
-}
-
-cudaError_t launch_mode_amp(const double* re, const double* im, int nx, int nz, int k, double* colbuf,
-                            const double* weight, double* out, cudaStream_t s) {
-  mode_amp_kernel<<<(nx + 127) / 128, 128, 0, s>>>(re, im, nx, nz, k, colbuf);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  mode_amp_final_kernel<<<1, 32, 0, s>>>(colbuf, weight, nx, nz, out);
-  return cudaGetLastError();
-}
-
 }  // namespace ymkh

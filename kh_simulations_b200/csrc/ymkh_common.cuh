@@ -232,9 +232,11 @@ cudaError_t launch_band(const ArrayList& arrs, int narr, const double* W, int ld
                         double inv2, cudaStream_t s);
 cudaError_t launch_twiddles(double* W, int nz, int lo, int hi, int ldw, cudaStream_t s);
 cudaError_t launch_twiddles_f32(float* c, float* sn, int nz, int lo, int hi, cudaStream_t s);
-cudaError_t launch_energy(const State& st, size_t N, double* part, double* out, cudaStream_t s);
+// part: 2 * energy_nparts(N) doubles.  out may be pinned host memory; with err, out[1] = the error word.
+cudaError_t launch_energy(const State& st, size_t N, double* part, double* out, const unsigned* err, cudaStream_t s);
 int energy_nparts(size_t N);
-cudaError_t launch_mode_amp(const double* re, const double* im, int nx, int nz, int k, double* colbuf,
+size_t mode_amp_scratch(int nx, int nz);  // doubles
+cudaError_t launch_mode_amp(const double* re, const double* im, int nx, int nz, int k, double* scratch,
                             const double* weight, double* out, cudaStream_t s);
 // State snapshots written by host threads (ymkh_snapshot.cu).
 class SnapshotQueue;
@@ -244,7 +246,7 @@ int snapshot_submit(SnapshotQueue* q, const State& st, int nx, int nz, double dx
                     int format, cudaStream_t s, std::string& err);
 int snapshot_wait(SnapshotQueue* q, std::string& err);
 // Non-Abelian Gauss law residual sums (ymkh_diag.cu); part holds
-// gauss_nparts(N) * YMKH_GAUSS_NOUT * 2 doubles, out YMKH_GAUSS_NOUT.
+// gauss_nparts(N) * YMKH_GAUSS_NOUT * 2 doubles, out YMKH_GAUSS_NOUT (it may be pinned host memory).
 int gauss_nparts(size_t N);
 cudaError_t launch_gauss(const State& st, int nx, int nz, double dx, double dz, double alpha, double* part,
                          double* out, cudaStream_t s);

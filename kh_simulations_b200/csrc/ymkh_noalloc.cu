@@ -99,7 +99,7 @@ extern "C" int ymkh_energy_noalloc(double* const* state, int nx, int nz, double*
     st.a[i] = state[12 + i];
     st.b[i] = state[18 + i];
   }
-  e = launch_energy(st, N, part, dev_out, (cudaStream_t)stream);
+  e = launch_energy(st, N, part, dev_out, nullptr, (cudaStream_t)stream);
   if (e != cudaSuccess) {
     char msg[200];
     snprintf(msg, sizeof msg, "ymkh_energy_noalloc: energy kernels: %s", cudaGetErrorString(e));
