@@ -149,7 +149,7 @@ struct ymkh_ctx {
   unsigned* derr = nullptr; // device error word of the bounded in-kernel waits
   // Tables of the kernels, uploaded in stream order by the next step call.
   struct Tables {
-    TensorMap maps[2 * kFctMaps];  // kFctMaps of buffer 0, then of buffer 1
+    TensorMap maps[2 * kMaps];     // kMaps of buffer 0, then of buffer 1
     RunDesc desc[2];               // run descriptors for start buffer 0 and 1
     ColDesc col[2];                // column stages writing buffer 0 and buffer 1
   };
@@ -358,12 +358,17 @@ RunDesc make_desc(const ymkh_ctx* c, int start, int tb, int fct_item0, int mx_it
   d.fct_bulk = (c->aligned16 && fct_bulk_ok(c->sp, tb)) ? kAlignedRowLoad : (int)LOAD_ELEM;
   if (tb == 128 && d.fct_bulk != LOAD_ELEM && c->boxed) {
     d.fct_bulk = LOAD_BOX;
-    d.maps = c->dev->maps + kFctMaps * start;
+    d.maps = c->dev->maps + kMaps * start;
   }
   d.mx_nstrips = maxwell_nstrips(c->nx);
   d.mx_seg = c->mx_seg;
   d.mx_item0 = mx_item0;
   d.mx_bulk = (c->aligned16 && maxwell_bulk_ok(c->sp)) ? kAlignedRowLoad : (int)LOAD_ELEM;
+  if (d.mx_bulk != LOAD_ELEM && c->boxed) {
+    d.mx_bulk = LOAD_BOX;
+    d.mx_fluid = c->dev->maps + kMaps * (1 - start) + kFctMaps;
+    d.mx_field = c->dev->maps + kMaps * start + kFctMaps;
+  }
   if (c->xscratch)
     for (int i = 0; i < 6; ++i) {
       d.xsw.a[i] = c->xscratch + (size_t)i * c->N;
@@ -389,7 +394,7 @@ int ensure_xscratch(ymkh_ctx* c) {
 int items_fct(const RunDesc& d, int nz) { return d.fct_nstrips * ((nz + d.fct_seg - 1) / d.fct_seg); }
 int items_mx(const RunDesc& d, int nz) { return d.mx_nstrips * ((nz + d.mx_seg - 1) / d.mx_seg); }
 
-// Tensor maps of both buffers for the FCT's TMA boxes: [array][z][x] with the
+// Tensor maps of both buffers for the kernels' TMA boxes: [array][z][x] with the
 // distance between arrays as the outer stride, which needs the 24 arrays of a
 // buffer evenly spaced in the state's order (a [24, NZ, NX] tensor, or the
 // library's own buffer).  Other layouts, odd NX and unaligned arrays keep the
@@ -499,9 +504,10 @@ int upload_desc(ymkh_ctx* c) {
   if (!c->dev) CK(cudaMalloc(&c->dev, sizeof(ymkh_ctx::Tables)), "cudaMalloc run tables");
   { int rc = ensure_xscratch(c); if (rc) return rc; }
   c->boxed = c->aligned16 && c->nx >= kFctBoxWidth;
-  constexpr int arrays[kFctMaps] = {12, 9, 1, 12, 9}, width[kFctMaps] = {kFctBoxWidth, kFctBoxWidth, kFctBoxWidth, 4, 4};
-  for (int k = 0; k < 2 * kFctMaps && c->boxed; ++k)
-    c->boxed = encode_box(&c->host.maps[k], c->buf[k / kFctMaps], c->nx, c->nz, arrays[k % kFctMaps], width[k % kFctMaps]);
+  const int arrays[kMaps] = {12, 9, 1, 12, 9, 12};
+  const int width[kMaps] = {kFctBoxWidth, kFctBoxWidth, kFctBoxWidth, 4, 4, maxwell_box_width()};
+  for (int k = 0; k < 2 * kMaps && c->boxed; ++k)
+    c->boxed = encode_box(&c->host.maps[k], c->buf[k / kMaps], c->nx, c->nz, arrays[k % kMaps], width[k % kMaps]);
   RunDesc* h = c->host.desc;
   h[0] = make_desc(c, 0, c->fct_tx, 0, 0);
   h[1] = make_desc(c, 1, c->fct_tx, 0, 0);

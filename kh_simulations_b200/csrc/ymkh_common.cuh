@@ -315,15 +315,18 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned by
                "l"(src), "r"(bytes), "r"(b)
                : "memory");
 }
-constexpr int kFctMaps = 5;  // tensor maps of a state buffer: 128-wide boxes of 12, 9 and 1 arrays, 4-wide boxes of 12 and 9
+// tensor maps of a state buffer: the FCT's 128-wide boxes of 12, 9 and 1 arrays
+// and 4-wide boxes of 12 and 9, then the Maxwell kernel's box of 12
+constexpr int kFctMaps = 5, kMaps = 6;
 // A TMA tensor map as the kernels see it (128 opaque bytes, encoded on the host).
 struct alignas(64) TensorMap {
   unsigned char bytes[128];
 };
 // Makes tensor maps written to global memory by the host visible to the TMA unit.
+template <int N = 1>
 __device__ __forceinline__ void tensormap_acquire(const TensorMap* m) {
 #pragma unroll
-  for (int k = 0; k < kFctMaps; ++k)
+  for (int k = 0; k < N; ++k)
     asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(m + k) : "memory");
 }
 // One box of a [array][z][x] tensor map to shared memory.  x must be even
@@ -364,7 +367,7 @@ namespace ymkh {
 enum RowLoad : int {
   LOAD_ELEM = 0,    // per-element 8-byte cp.async through an x index table (walls, odd nx)
   LOAD_BULK_ALL = 3, // TMA bulk row copies, one per thread spread over all warps
-  LOAD_BOX = 4       // FCT: evenly spaced arrays, a row is a few TMA boxes
+  LOAD_BOX = 4       // evenly spaced arrays, a row is a few TMA boxes
 };
 
 // One run of a batch as the fused kernels see it: its start-of-step and
@@ -375,7 +378,10 @@ struct RunDesc {
   State in;
   State out;
   State xsw;  // x-swept fluid scratch of the split FCT form (fluid arrays only)
-  const TensorMap* maps;  // kFctMaps tensor maps of `in` (device memory; LOAD_BOX only)
+  // tensor maps in device memory (LOAD_BOX only): kFctMaps of `in` for the FCT,
+  // Maxwell's of `out` (the new fluid) and of `in` (the old fields)
+  const TensorMap* maps;
+  const TensorMap *mx_fluid, *mx_field;
   StepParams p;
   int fct_nstrips, fct_seg, fct_item0, fct_bulk;
   int mx_nstrips, mx_seg, mx_item0, mx_bulk;
@@ -425,6 +431,7 @@ __device__ __forceinline__ void load_desc(RunDesc* dst, const RunDesc* src) {
 cudaError_t launch_fct_table(const RunTable& T, int tb, int grid_ctas, cudaStream_t s);
 cudaError_t launch_maxwell_table(const RunTable& T, int grid_ctas, cudaStream_t s);
 constexpr int kFctBoxWidth = 128;  // columns of the FCT's TMA boxes
+int maxwell_box_width();           // and of the Maxwell kernel's
 int fct_nstrips(int nx, int tb);
 int maxwell_nstrips(int nx);
 int fct_bulk_ok(const StepParams& p, int tb);

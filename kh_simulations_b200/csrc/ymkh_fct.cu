@@ -850,7 +850,7 @@ __global__ void __launch_bounds__(F2_NT, 1) fct_strip_kernel(const __grid_consta
       // x = nx in the last) come as three narrow boxes and are put in their
       // places when the row is there.  With warm_T such a strip copies row by row.
       const TensorMap* const maps = rd.maps;  // boxes of 12, 9 and 1 arrays; 4-wide boxes of 12 and 9 arrays
-      if (box && htid == 0) tensormap_acquire(maps);
+      if (box && htid == 0) tensormap_acquire<kFctMaps>(maps);
       const bool patch_l = x0 == 0, patch = box && c.edge;
       const int patch_q = patch_l ? 0 : nx - (x0 - 4);  // position of the first wrapped column
       if (!bulk) xtab[q] = xmap(x0 - 4 + q, nx, p.periodic_x);

@@ -45,13 +45,17 @@ constexpr int MX_NT = YMKH_MX_NT;    // threads per CTA: [0,NT/2) Ex / By half, 
 constexpr int MX_NST = YMKH_MX_NST;  // stage ring depth: rows q-1, q in use, NST-2 rows in flight
 constexpr int MX_W = MX_TX + 4;  // stage row: position s <-> x = x0 - 2 + s (66: even)
 
-// stage offsets in rows of MX_W doubles (every array staged over the full row)
-constexpr int MS_FL = 0;   // 12 fluid arrays
-constexpr int MS_BY = 12;  // By1..3
-constexpr int MS_AZ = 15;  // Az1..3
-constexpr int MS_EX = 18;  // Ex1..3
-constexpr int MS_EZ = 21;  // Ez1..3
-constexpr int MS_SIZE = 24;
+// Stage offsets in doubles; an array's row is MX_W doubles.  The fluid and the
+// field half each start on 128 bytes (the destination of a TMA box).
+constexpr int MS_HALF = (12 * MX_W + 15) / 16 * 16;
+constexpr int MS_FL = 0;                      // 12 fluid arrays
+constexpr int MS_EX = MS_HALF;                // the fields in the state's order: Ex1..3
+constexpr int MS_EZ = MS_HALF + 3 * MX_W;     // Ez1..3
+constexpr int MS_BY = MS_HALF + 6 * MX_W;     // By1..3
+constexpr int MS_AZ = MS_HALF + 9 * MX_W;     // Az1..3
+constexpr int MS_STAGE = 2 * MS_HALF;
+constexpr int MS_ARRAYS = 24;
+__device__ __forceinline__ int ms_row(int a) { return a < 12 ? a * MX_W : MS_HALF + (a - 12) * MX_W; }
 
 // work rows: per-cell velocities [2 rows][beam][px/n, pz/n], new Ex [2 rows][3], new Ez [3]
 constexpr int MW_V = 0;
@@ -62,7 +66,7 @@ constexpr int MW_SIZE = 17;
 }  // namespace
 
 constexpr size_t maxwell_smem_bytes() {
-  return (size_t)MX_W * sizeof(double) * (MX_NST * MS_SIZE + MW_SIZE) + (size_t)MX_W * sizeof(int) +
+  return sizeof(double) * ((size_t)MX_NST * MS_STAGE + (size_t)MX_W * MW_SIZE) + (size_t)MX_W * sizeof(int) +
          (size_t)8 * MX_NST + 16;
 }
 
@@ -71,9 +75,10 @@ __global__ void __launch_bounds__(MX_NT, YMKH_MX_MINB)
   constexpr int TX = MX_TX, NV = MX_NV, W = MX_W, NST = MX_NST, NT = MX_NT;
   static_assert(2 * NV <= NT && TX <= NT / 2 && NV <= NT / 2, "one item per thread per phase");
   static_assert(W % 2 == 0 && TX % 2 == 0, "even strip origin and row length for 16-byte row copies");
-  extern __shared__ __align__(16) double smem[];
+  extern __shared__ __align__(128) double smem[];
+  static_assert(MS_STAGE % 16 == 0 && MS_HALF % 16 == 0, "TMA box destinations on 128 bytes");
   double* const stage = smem;
-  double* const wk = smem + (size_t)NST * MS_SIZE * W;
+  double* const wk = smem + (size_t)NST * MS_STAGE;
   int* const xtab = reinterpret_cast<int*>(wk + (size_t)MW_SIZE * W);
   uint64_t* const bars = reinterpret_cast<uint64_t*>(
       (reinterpret_cast<uintptr_t>(xtab + W) + 15) & ~static_cast<uintptr_t>(15));
@@ -103,7 +108,7 @@ __global__ void __launch_bounds__(MX_NT, YMKH_MX_MINB)
     __syncthreads();
     const int nx = p.nx, nz = p.nz;
     const bool wall = !p.periodic_x;
-    const bool bulk = rd.mx_bulk == LOAD_BULK_ALL;  // TMA bulk rows on mbarriers (else per-element cp.async)
+    const bool bulk = rd.mx_bulk != LOAD_ELEM;  // TMA rows on mbarriers (else per-element cp.async)
     const double dt = p.dt, c2 = p.c2, al = p.alpha, e0 = p.eps0;
     // c = eps_0 = 1 (ymgpu2d/main_ym.cu:69): 1*x and x/1 are exact, so the
     // products and quotients by them can be skipped without changing a bit
@@ -113,34 +118,47 @@ __global__ void __launch_bounds__(MX_NT, YMKH_MX_MINB)
     const int zs = (local / rd.mx_nstrips) * rd.mx_seg;
     const int ze = min(nz, zs + rd.mx_seg);
 
+    // Evenly spaced arrays: a row is two TMA boxes, of the 12 new fluid and the
+    // 12 old field arrays, where the strip's window does not wrap.
+    const bool box = rd.mx_bulk == LOAD_BOX && x0 >= 2 && x0 - 2 + W <= nx;
+    if (box && tid == 0) {
+      tensormap_acquire(rd.mx_fluid);
+      tensormap_acquire(rd.mx_field);
+    }
+
     for (int i = tid; i < W; i += NT) xtab[i] = xmap(x0 - 2 + i, nx, p.periodic_x);
     __syncthreads();
 
     auto issue_row = [&](int q) {
       const int s = (int)(issued % NST);
-      double* sb = stage + (size_t)s * MS_SIZE * W;
+      double* sb = stage + (size_t)s * MS_STAGE;
       const size_t ro = (size_t)zwrap(q, nz) * nx;
       auto arr = [&](int a) -> const double* {
         if (a < 12) return (a < 6) ? fluid_new.a[a] : fluid_new.b[a - 6];
-        const int kind = (a - 12) / 3, c = (a - 12) % 3;
-        return (kind == 0) ? fields_old.f[BY1 + c]
-               : (kind == 1) ? fields_old.f[AZ1 + c]
-               : (kind == 2) ? fields_old.f[EX1 + c]
-                             : fields_old.f[EZ1 + c];
+        return fields_old.f[a - 12];
       };
-      if (bulk) {
+      if (box) {
+        if (tid == 0) {
+          const int z = zwrap(q, nz);
+          mbar_expect_tx(&bars[s], (unsigned)(MS_ARRAYS * W * 8));
+          if (dbg_ok(z >= 0 && z < nz, T.err)) {
+            box_g2s(sb + MS_FL, rd.mx_fluid, x0 - 2, z, 12, &bars[s]);
+            box_g2s(sb + MS_EX, rd.mx_field, x0 - 2, z, 0, &bars[s]);
+          }
+        }
+      } else if (bulk) {
         // one row copy per thread, spread over the warps (lane-major); early
         // completions only drive the transaction count negative before
         // thread 0's arrival arms the phase
-        if (tid == 0) mbar_expect_tx(&bars[s], (unsigned)(MS_SIZE * W * 8));
+        if (tid == 0) mbar_expect_tx(&bars[s], (unsigned)(MS_ARRAYS * W * 8));
         const int a = (tid & 31) * (NT / 32) + (tid >> 5);
-        if (a < MS_SIZE && dbg_ok(zwrap(q, nz) >= 0 && zwrap(q, nz) < nz && W <= nx && (x0 - 2) % 2 == 0, T.err))
-          bulk_row_periodic(sb + a * W, arr(a) + ro, x0 - 2, W, nx, &bars[s]);
+        if (a < MS_ARRAYS && dbg_ok(zwrap(q, nz) >= 0 && zwrap(q, nz) < nz && W <= nx && (x0 - 2) % 2 == 0, T.err))
+          bulk_row_periodic(sb + ms_row(a), arr(a) + ro, x0 - 2, W, nx, &bars[s]);
       } else {
-        for (int i = tid; i < MS_SIZE * W; i += NT) {
+        for (int i = tid; i < MS_ARRAYS * W; i += NT) {
           const int a = i / W, k = i - a * W;
           if (dbg_ok(zwrap(q, nz) >= 0 && zwrap(q, nz) < nz && xtab[k] >= 0 && xtab[k] < nx, T.err))
-            cp_async8(sb + a * W + k, arr(a) + ro + xtab[k]);
+            cp_async8(sb + ms_row(a) + k, arr(a) + ro + xtab[k]);
         }
         cp_async_commit();
       }
@@ -168,14 +186,14 @@ __global__ void __launch_bounds__(MX_NT, YMKH_MX_MINB)
       ++consumed;
       if (q + NST - 2 <= q_last) issue_row(q + NST - 2);
       else if (!bulk) cp_async_commit();
-      const double* sb = stage + (size_t)s * MS_SIZE * W;      // row q
-      const double* sp = stage + (size_t)sprev * MS_SIZE * W;  // row q-1
+      const double* sb = stage + (size_t)s * MS_STAGE;      // row q
+      const double* sp = stage + (size_t)sprev * MS_STAGE;  // row q-1
       const int rq = q & 1, rp = (q - 1) & 1;
 
       // ---- 1: per-cell velocities of row q at x in [x0, x0+TX] (YM_Physics.cu:22-25, 38-41)
       if (tid < 2 * NV) {
         const int b = tid / NV, k = 2 + (tid - b * NV);
-        const double* fl = sb + (size_t)(MS_FL + 6 * b) * W;
+        const double* fl = sb + MS_FL + 6 * b * W;
         const double n = fmax(fl[FN * W + k], 1e-10);
         wk[(MW_V + rq * 4 + b * 2 + 0) * W + k] = fl[FPX * W + k] / n;
         wk[(MW_V + rq * 4 + b * 2 + 1) * W + k] = fl[FPZ * W + k] / n;
@@ -188,22 +206,22 @@ __global__ void __launch_bounds__(MX_NT, YMKH_MX_MINB)
         double nq[2][3], vxr[2];
 #pragma unroll
         for (int b = 0; b < 2; ++b) {
-          const double* fl = sb + (size_t)(MS_FL + 6 * b) * W;
+          const double* fl = sb + MS_FL + 6 * b * W;
           const double n0 = fl[FN * W + k], n1 = fl[FN * W + k + 1];
           vxr[b] = 0.5 * (wk[(MW_V + rq * 4 + b * 2) * W + k] + wk[(MW_V + rq * 4 + b * 2) * W + k + 1]);
 #pragma unroll
           for (int a = 0; a < 3; ++a) nq[b][a] = 0.5 * (n0 * fl[(FQ1 + a) * W + k] + n1 * fl[(FQ1 + a) * W + k + 1]);
         }
-        const double by1 = sb[(MS_BY + 0) * W + k], by2 = sb[(MS_BY + 1) * W + k], by3 = sb[(MS_BY + 2) * W + k];
-        const double dz3[3] = {div_rn(by1 - sp[(MS_BY + 0) * W + k], p.dz, p.rdz), div_rn(by2 - sp[(MS_BY + 1) * W + k], p.dz, p.rdz),
-                               div_rn(by3 - sp[(MS_BY + 2) * W + k], p.dz, p.rdz)};
-        const double a1 = sb[(MS_AZ + 0) * W + k], a2 = sb[(MS_AZ + 1) * W + k], a3 = sb[(MS_AZ + 2) * W + k];
+        const double by1 = sb[MS_BY + 0 * W + k], by2 = sb[MS_BY + 1 * W + k], by3 = sb[MS_BY + 2 * W + k];
+        const double dz3[3] = {div_rn(by1 - sp[MS_BY + 0 * W + k], p.dz, p.rdz), div_rn(by2 - sp[MS_BY + 1 * W + k], p.dz, p.rdz),
+                               div_rn(by3 - sp[MS_BY + 2 * W + k], p.dz, p.rdz)};
+        const double a1 = sb[MS_AZ + 0 * W + k], a2 = sb[MS_AZ + 1 * W + k], a3 = sb[MS_AZ + 2 * W + k];
         const double kx[3] = {a2 * by3 - a3 * by2, a3 * by1 - a1 * by3, a1 * by2 - a2 * by1};
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
           const double jx = -(nq[0][a] * vxr[0] + nq[1][a] * vxr[1]);
           const double rhs = unit ? (-dz3[a] - al * kx[a]) - jx : c2 * (-dz3[a] - al * kx[a]) - jx / e0;
-          wk[(MW_EX + rq * 3 + a) * W + k] = sb[(MS_EX + a) * W + k] + dt * rhs;
+          wk[(MW_EX + rq * 3 + a) * W + k] = sb[MS_EX + a * W + k] + dt * rhs;
         }
       } else {
         // ---- 2b: Ampère for Ez on row q-1, columns [x0, x0+TX]
@@ -213,8 +231,8 @@ __global__ void __launch_bounds__(MX_NT, YMKH_MX_MINB)
           double nqz[2][3], vzt[2];
 #pragma unroll
           for (int b = 0; b < 2; ++b) {
-            const double* f0 = sp + (size_t)(MS_FL + 6 * b) * W;
-            const double* f1 = sb + (size_t)(MS_FL + 6 * b) * W;
+            const double* f0 = sp + MS_FL + 6 * b * W;
+            const double* f1 = sb + MS_FL + 6 * b * W;
             const double n0 = f0[FN * W + k], n1 = f1[FN * W + k];
             vzt[b] = 0.5 * (wk[(MW_V + rp * 4 + b * 2 + 1) * W + k] + wk[(MW_V + rq * 4 + b * 2 + 1) * W + k]);
 #pragma unroll
@@ -225,9 +243,9 @@ __global__ void __launch_bounds__(MX_NT, YMKH_MX_MINB)
 #pragma unroll
           for (int a = 0; a < 3; ++a) {
             const double jz = -(nqz[0][a] * vzt[0] + nqz[1][a] * vzt[1]);
-            const double by = sp[(MS_BY + a) * W + k];
-            const double dbx = div_rn(by - sp[(MS_BY + a) * W + k - 1], p.dx, p.rdx);
-            const double ez0 = wz ? 0.0 : sp[(MS_EZ + a) * W + k];
+            const double by = sp[MS_BY + a * W + k];
+            const double dbx = div_rn(by - sp[MS_BY + a * W + k - 1], p.dx, p.rdx);
+            const double ez0 = wz ? 0.0 : sp[MS_EZ + a * W + k];
             wk[(MW_EZ + a) * W + k] = ez0 + dt * (unit ? dbx - jz : c2 * dbx - jz / e0);
           }
         }
@@ -261,7 +279,7 @@ __global__ void __launch_bounds__(MX_NT, YMKH_MX_MINB)
         if (tid < NT / 2) {
           double az[3];
 #pragma unroll
-          for (int a = 0; a < 3; ++a) az[a] = sp[(MS_AZ + a) * W + k];
+          for (int a = 0; a < 3; ++a) az[a] = sp[MS_AZ + a * W + k];
           if (!p.freeze_az1) az[0] = az[0] - dt * ez[0];
           az[1] = az[1] - dt * ez[1];
           az[2] = az[2] - dt * ez[2];
@@ -271,7 +289,7 @@ __global__ void __launch_bounds__(MX_NT, YMKH_MX_MINB)
           for (int a = 0; a < 3; ++a) {
             const double dex = div_rn(wk[(MW_EX + rq * 3 + a) * W + k] - ex[a], p.dz, p.rdz);
             const double dez = div_rn(wk[(MW_EZ + a) * W + k + 1] - ez[a], p.dx, p.rdx);
-            out.f[BY1 + a][gi] = sp[(MS_BY + a) * W + k] - dt * (dex - dez - al * kk[a]);
+            out.f[BY1 + a][gi] = sp[MS_BY + a * W + k] - dt * (dex - dez - al * kk[a]);
             out.f[AZ1 + a][gi] = az[a];
           }
         } else {
@@ -297,6 +315,8 @@ int maxwell_ctas_per_sm() {
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, maxwell_fused_kernel, MX_NT, maxwell_smem_bytes());
   return n;
 }
+
+int maxwell_box_width() { return MX_W; }
 
 int maxwell_nstrips(int nx) { return (nx + MX_TX - 1) / MX_TX; }
 
