@@ -61,6 +61,7 @@ struct NvtxRange {
   } while (0)
 
 constexpr int MAX_BANDS = kMaxBands;
+constexpr int kMaxFctCtas = 512;
 
 // Pages of pinned host memory that the diagnostics' last kernels write their
 // results to, one slot of 32 doubles per context: reading a result back is
@@ -152,6 +153,7 @@ struct ymkh_ctx {
     TensorMap maps[2 * kMaps];     // kMaps of buffer 0, then of buffer 1
     RunDesc desc[2];               // run descriptors for start buffer 0 and 1
     ColDesc col[2];                // column stages writing buffer 0 and buffer 1
+    int fct_first[kMaxFctCtas + 1];  // items of the 128-wide FCT's CTAs
   };
   Tables host{};              // host copy
   Tables* dev = nullptr;      // device copy
@@ -391,6 +393,8 @@ int ensure_xscratch(ymkh_ctx* c) {
   return 0;
 }
 
+// CTAs of an FCT launch (launch_fct_table).
+int fct_ctas(int items, int grid) { return std::max(1, std::min(std::min(items, grid), kMaxFctCtas)); }
 int items_fct(const RunDesc& d, int nz) { return d.fct_nstrips * ((nz + d.fct_seg - 1) / d.fct_seg); }
 int items_mx(const RunDesc& d, int nz) { return d.mx_nstrips * ((nz + d.mx_seg - 1) / d.mx_seg); }
 
@@ -497,6 +501,52 @@ bool col_fused_alone(const ymkh_ctx* c) {
   return stages >= 2 || (c->nb && c->nz <= 128);
 }
 
+// How the 128-wide FCT's items (strip-major segments) are cut into one
+// contiguous block per CTA.  The launch lasts as long as its slowest CTA, so
+// the blocks are equal in cost, not in rows: in units of a fifth of an inner
+// strip's row, a row of a strip whose window wraps takes 6 (its wrapped columns
+// are put in place separately: 480 against 400 thousand cycles for 131 rows),
+// and entering a strip kFctEntry more (its pipeline's fill).  With few rows per
+// CTA the cut is by rows: there a whole row decides.  FCT of one step, against
+// equal rows: 3.42 -> 3.12 ms at 4096 x 8192, 252 -> 227 us at 1024 x 2048
+// (entry 0, 20, 60: 236, 229, 227; edge row 7: 230).
+struct StripRun {
+  int nstrips, nseg, seg;
+  bool box;
+};
+constexpr int kFctEntry = 40, kFctEdgeRow = 6, kFctInnerRow = 5, kFctEvenBelow = 16;
+void cut_fct(const std::vector<StripRun>& runs, int grid, int* first) {
+  long long items = 0, rows = 0, cost = 0;
+  auto row_cost = [](const StripRun& r, int s) { return r.box && (s == 0 || s == r.nstrips - 1) ? kFctEdgeRow : kFctInnerRow; };
+  for (const StripRun& r : runs) {
+    items += (long long)r.nstrips * r.nseg;
+    rows += (long long)r.nstrips * r.nseg * r.seg;
+    for (int s = 0; s < r.nstrips; ++s) cost += kFctEntry + (long long)r.nseg * r.seg * row_cost(r, s);
+  }
+  first[0] = 0;
+  if (rows < (long long)kFctEvenBelow * grid) {
+    const long long per = (items + grid - 1) / std::max(grid, 1);
+    for (int b = 1; b <= grid; ++b) first[b] = (int)std::min(items, b * per);
+    return;
+  }
+  int b = 1;
+  long long at = 0, item = 0;  // cost and items ahead of the strip
+  for (const StripRun& r : runs)
+    for (int s = 0; s < r.nstrips; ++s) {
+      const long long unit = (long long)r.seg * row_cost(r, s), end = at + kFctEntry + r.nseg * unit;
+      for (; b < grid && cost * b / grid < end; ++b) {
+        const long long into = cost * b / grid - at - kFctEntry;
+        first[b] = (int)(item + (into <= 0 ? 0 : std::min<long long>(r.nseg, (into + unit / 2) / unit)));
+      }
+      at = end;
+      item += r.nseg;
+    }
+  for (; b <= grid; ++b) first[b] = (int)items;
+}
+StripRun strip_run(const RunDesc& d, int nz) {
+  return {d.fct_nstrips, (nz + d.fct_seg - 1) / d.fct_seg, d.fct_seg, d.fct_bulk == LOAD_BOX};
+}
+
 // Device descriptors of this run for both start buffers (single-run tables).
 int upload_desc(ymkh_ctx* c) {
   c->desc_ok = false;
@@ -513,6 +563,7 @@ int upload_desc(ymkh_ctx* c) {
   h[1] = make_desc(c, 1, c->fct_tx, 0, 0);
   for (int i = 0; i < 2; ++i) h[i].fx_item0 = h[i].fz_item0 = 0;
   c->fct_items = items_fct(h[0], c->nz);
+  if (c->fct_tx == 128) cut_fct({strip_run(h[0], c->nz)}, fct_ctas(c->fct_items, c->fct_grid), c->host.fct_first);
   c->mx_items = items_mx(h[0], c->nz);
   c->fx_items = items_fx(h[0], c->nz);
   c->fz_items = items_fz(h[0], c->nz);
@@ -617,7 +668,7 @@ bool has_column_stages(const ymkh_ctx* c) {
 // One reference iteration from buffer c->cur into buffer 1 - c->cur.
 int step_once(ymkh_ctx* c, cudaStream_t s) {
   { int rc = flush_desc(c, s); if (rc) return rc; }
-  RunTable T{c->dev->desc + c->cur, 1, c->fct_items, c->mx_items, c->derr, c->fx_items, c->fz_items, 1};
+  RunTable T{c->dev->desc + c->cur, 1, c->fct_items, c->mx_items, c->derr, c->fx_items, c->fz_items, 1, c->dev->fct_first};
   mark(c, ST_FCT, s);
   {
     NvtxRange r("ymkh fct");
@@ -625,7 +676,7 @@ int step_once(ymkh_ctx* c, cudaStream_t s) {
       CK(launch_fct_split_table(T, c->fx_grid, c->fz_grid, s), "fct_x/fct_z kernels");
       g_launches++;
     } else {
-      CK(launch_fct_table(T, c->fct_tx, c->fct_grid, s), "fct_fused_kernel");
+      CK(launch_fct_table(T, c->fct_tx, fct_ctas(c->fct_items, c->fct_grid), s), "fct_fused_kernel");
     }
   }
   mark(c, ST_MAXWELL, s);
@@ -1086,6 +1137,7 @@ struct ymkh_batch {
   // members whose column stages run fused, grouped by NZ (one launch a group)
   struct ColGroup { int nz, first, n, items; size_t smem; };
   ColDesc* dcol = nullptr;   // [2][cap]
+  int* dfirst = nullptr;     // items of the 128-wide FCT's CTAs
   std::vector<ColGroup> col;
   std::vector<char> col_member;    // whether the member is in one of the groups
   std::vector<unsigned> versions;  // of the members' descriptors when the tables were built
@@ -1128,6 +1180,7 @@ int batch_build(ymkh_batch* b, cudaStream_t s) {
     b->cap = cap;
   }
   std::vector<RunDesc> h(2 * (size_t)std::max(n, 1));
+  std::vector<StripRun> strips;
   std::vector<MxGrid> mg;
   for (const ymkh_ctx* c : b->runs) mg.push_back({c->nz, maxwell_nstrips(c->nx)});
   const int mx_seg = pick_mx_segment(mg.data(), n, b->mx_grid);
@@ -1157,6 +1210,7 @@ int batch_build(ymkh_batch* b, cudaStream_t s) {
     d0.mx_item0 = d1.mx_item0 = m0;
     h[i] = d0;
     h[n + i] = d1;
+    strips.push_back(strip_run(d0, c->nz));
     f0 += items_fct(d0, c->nz);
     m0 += items_mx(d0, c->nz);
   }
@@ -1203,6 +1257,12 @@ int batch_build(ymkh_batch* b, cudaStream_t s) {
   }
   for (int p = 0; p < 2 && !order.empty(); ++p)
     CK(upload_table(b->dcol + (size_t)p * b->cap, hc[p].data(), hc[p].size() * sizeof(ColDesc), s), "upload batch column table");
+  if (n) {
+    std::vector<int> first(kMaxFctCtas + 1);
+    cut_fct(strips, fct_ctas(b->fct_items, b->fct_grid), first.data());
+    if (!b->dfirst) CK(cudaMalloc(&b->dfirst, first.size() * sizeof(int)), "cudaMalloc batch FCT blocks");
+    CK(upload_table(b->dfirst, first.data(), first.size() * sizeof(int), s), "upload batch FCT blocks");
+  }
   b->parity = 0;
   b->dirty = false;
   batch_drop_graph(b);
@@ -1212,11 +1272,11 @@ int batch_build(ymkh_batch* b, cudaStream_t s) {
 int batch_step_once(ymkh_batch* b, cudaStream_t s) {
   const int n = (int)b->runs.size();
   if (!n) return 0;
-  RunTable T{b->ddesc + (size_t)b->parity * b->cap, n, b->fct_items, b->mx_items, b->derr, b->fx_items, b->fz_items, 1};
+  RunTable T{b->ddesc + (size_t)b->parity * b->cap, n, b->fct_items, b->mx_items, b->derr, b->fx_items, b->fz_items, 1, b->dfirst};
   if (b->fct_mode == YMKH_FCT_SPLIT)
     CK(launch_fct_split_table(T, b->fx_grid, b->fz_grid, s), "fct_x/fct_z kernels (batch)");
   else
-    CK(launch_fct_table(T, b->tb, b->fct_grid, s), "fct_fused_kernel (batch)");
+    CK(launch_fct_table(T, b->tb, fct_ctas(b->fct_items, b->fct_grid), s), "fct_fused_kernel (batch)");
   CK(launch_maxwell_table(T, b->mx_grid, s), "maxwell_fused_kernel (batch)");
   g_launches += 2;
   // column stages: one launch per NZ of the fused ones, the others per member;
@@ -1403,6 +1463,7 @@ int ymkh_batch_destroy(ymkh_batch* b) {
   batch_drop_graph(b);
   if (b->ddesc) cudaFree(b->ddesc);
   if (b->dcol) cudaFree(b->dcol);
+  if (b->dfirst) cudaFree(b->dfirst);
   if (b->derr) cudaFree(b->derr);
   for (int i = 0; i < ymkh_batch::kAux; ++i) {
     if (b->aux[i]) cudaStreamDestroy(b->aux[i]);

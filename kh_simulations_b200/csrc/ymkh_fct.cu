@@ -620,10 +620,8 @@ __global__ void __launch_bounds__(F2_NT, 1) fct_strip_kernel(const __grid_consta
   unsigned seq = 0;
   unsigned phase_bits = 0;  // per-barrier phase of the bulk path (one coefficient thread waits)
 
-  const bool contig = T.fct_contig != 0;
-  const int per = contig ? (T.fct_items + (int)gridDim.x - 1) / (int)gridDim.x : 0;
-  const int i_beg = contig ? (int)blockIdx.x * per : (int)blockIdx.x;
-  const int i_end = contig ? min(T.fct_items, i_beg + per) : T.fct_items;
+  // this CTA's items: a contiguous block, cut by cost on the host
+  const int i_beg = T.fct_first[blockIdx.x], i_end = T.fct_first[blockIdx.x + 1];
 
   // The piece that starts at an item: its run, strip and rows.  Every thread
   // calls it once per piece; the barriers also end the previous piece.
@@ -647,19 +645,10 @@ __global__ void __launch_bounds__(F2_NT, 1) fct_strip_kernel(const __grid_consta
     c.bulk = rd.fct_bulk != LOAD_ELEM;
     const int nseg = (nz + rd.fct_seg - 1) / rd.fct_seg;
     const int local = item - rd.fct_item0;
-    int strip;
-    if (contig) {
-      strip = local / nseg;
-      const int seg0 = local - strip * nseg;
-      c.next = min(i_end, rd.fct_item0 + (strip + 1) * nseg);  // past this piece's last segment
-      c.zs = seg0 * rd.fct_seg;
-      c.ze = min(nz, (seg0 + (c.next - item)) * rd.fct_seg);
-    } else {
-      strip = local % rd.fct_nstrips;
-      c.zs = (local / rd.fct_nstrips) * rd.fct_seg;
-      c.ze = min(nz, c.zs + rd.fct_seg);
-      c.next = item + (int)gridDim.x;
-    }
+    const int strip = local / nseg, seg0 = local - strip * nseg;
+    c.next = min(i_end, rd.fct_item0 + (strip + 1) * nseg);  // past this piece's last segment
+    c.zs = seg0 * rd.fct_seg;
+    c.ze = min(nz, (seg0 + (c.next - item)) * rd.fct_seg);
     c.x0 = strip * F2_O;
     c.edge = c.x0 == 0 || c.x0 - 4 + W > nx;
     c.box = rd.fct_bulk == LOAD_BOX && !(c.warm && c.edge);
