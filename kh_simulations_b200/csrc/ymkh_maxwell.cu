@@ -5,6 +5,14 @@
 // Ampère (YM_Physics.cu:70-113), potential (YM_Physics.cu:589-599) and
 // Faraday (YM_Physics.cu:120-151).  The currents are never stored.
 //
+// What bounds it: three CTA barriers a row and the FP64 chains between them, at
+// two CTAs of eight warps an SM (1.82 ms at 4096 x 8192, 5.2 TB/s of the 280 B
+// a cell; 139 us at 1024 x 2048).  Rows as TMA boxes, one reciprocal for both
+// velocities of a beam and no remainders in the row loop took it from 1.91 ms.
+// Strips whose window wraps still copy row by row (253 against 220 thousand
+// cycles for 61 rows); patching their wrapped columns into boxes cost a barrier
+// a row and more (1.96 ms).
+//
 // Layout: work items are (x-strip of TX columns, z-segment) pairs handed to
 // persistent CTAs round-robin; a CTA streams along z with the rows it needs
 // staged in shared memory NST-2 rows ahead (TMA bulk row copies, one per
@@ -97,8 +105,8 @@ __global__ void __launch_bounds__(MX_NT, YMKH_MX_MINB)
     for (int s = 0; s < NST; ++s) mbar_init(&bars[s], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  unsigned issued = 0, consumed = 0;
-  unsigned phase_bits = 0;  // per-stage mbarrier phase of the bulk path
+  int s_issue = 0, s_row = 0;  // ring slots of the next row to request and to use
+  unsigned phase_bits = 0;     // per-stage mbarrier phase of the bulk path
 
   for (int item = blockIdx.x; item < T.mx_items; item += gridDim.x) {
     __syncthreads();
@@ -130,16 +138,16 @@ __global__ void __launch_bounds__(MX_NT, YMKH_MX_MINB)
     __syncthreads();
 
     auto issue_row = [&](int q) {
-      const int s = (int)(issued % NST);
-      double* sb = stage + (size_t)s * MS_STAGE;
-      const size_t ro = (size_t)zwrap(q, nz) * nx;
+      const int s = s_issue;
+      double* sb = stage + s * MS_STAGE;
+      const int z = q < 0 ? q + nz : (q >= nz ? q - nz : q);
+      const size_t ro = (size_t)z * nx;
       auto arr = [&](int a) -> const double* {
         if (a < 12) return (a < 6) ? fluid_new.a[a] : fluid_new.b[a - 6];
         return fields_old.f[a - 12];
       };
       if (box) {
         if (tid == 0) {
-          const int z = zwrap(q, nz);
           mbar_expect_tx(&bars[s], (unsigned)(MS_ARRAYS * W * 8));
           if (dbg_ok(z >= 0 && z < nz, T.err)) {
             box_g2s(sb + MS_FL, rd.mx_fluid, x0 - 2, z, 12, &bars[s]);
@@ -152,17 +160,17 @@ __global__ void __launch_bounds__(MX_NT, YMKH_MX_MINB)
         // thread 0's arrival arms the phase
         if (tid == 0) mbar_expect_tx(&bars[s], (unsigned)(MS_ARRAYS * W * 8));
         const int a = (tid & 31) * (NT / 32) + (tid >> 5);
-        if (a < MS_ARRAYS && dbg_ok(zwrap(q, nz) >= 0 && zwrap(q, nz) < nz && W <= nx && (x0 - 2) % 2 == 0, T.err))
+        if (a < MS_ARRAYS && dbg_ok(z >= 0 && z < nz && W <= nx && (x0 - 2) % 2 == 0, T.err))
           bulk_row_periodic(sb + ms_row(a), arr(a) + ro, x0 - 2, W, nx, &bars[s]);
       } else {
         for (int i = tid; i < MS_ARRAYS * W; i += NT) {
           const int a = i / W, k = i - a * W;
-          if (dbg_ok(zwrap(q, nz) >= 0 && zwrap(q, nz) < nz && xtab[k] >= 0 && xtab[k] < nx, T.err))
+          if (dbg_ok(z >= 0 && z < nz && xtab[k] >= 0 && xtab[k] < nx, T.err))
             cp_async8(sb + ms_row(a) + k, arr(a) + ro + xtab[k]);
         }
         cp_async_commit();
       }
-      ++issued;
+      s_issue = s_issue == NST - 1 ? 0 : s_issue + 1;
     };
 
     // Rows q-1 and q are read in the same iteration, so NST-2 rows are in
@@ -173,8 +181,7 @@ __global__ void __launch_bounds__(MX_NT, YMKH_MX_MINB)
       else if (!bulk) cp_async_commit();
 
     for (int q = q_first; q <= q_last; ++q) {
-      const int s = (int)(consumed % NST);
-      const int sprev = (int)((consumed + NST - 1) % NST);
+      const int s = s_row, sprev = s_row == 0 ? NST - 1 : s_row - 1;
       if (bulk) {  // one thread polls the stage's mbarrier; the CTA barrier below
         // releases the others after it (no spinning by every thread)
         if (tid == 0) mbar_wait(&bars[s], (phase_bits >> s) & 1u, T.err);
@@ -183,11 +190,11 @@ __global__ void __launch_bounds__(MX_NT, YMKH_MX_MINB)
       else
         cp_async_wait<NST - 3>();
       __syncthreads();  // row q staged by every thread; row q-2's stage is free
-      ++consumed;
+      s_row = s_row == NST - 1 ? 0 : s_row + 1;
       if (q + NST - 2 <= q_last) issue_row(q + NST - 2);
       else if (!bulk) cp_async_commit();
-      const double* sb = stage + (size_t)s * MS_STAGE;      // row q
-      const double* sp = stage + (size_t)sprev * MS_STAGE;  // row q-1
+      const double* sb = stage + s * MS_STAGE;      // row q
+      const double* sp = stage + sprev * MS_STAGE;  // row q-1
       const int rq = q & 1, rp = (q - 1) & 1;
 
       // ---- 1: per-cell velocities of row q at x in [x0, x0+TX] (YM_Physics.cu:22-25, 38-41)
@@ -195,8 +202,10 @@ __global__ void __launch_bounds__(MX_NT, YMKH_MX_MINB)
         const int b = tid / NV, k = 2 + (tid - b * NV);
         const double* fl = sb + MS_FL + 6 * b * W;
         const double n = fmax(fl[FN * W + k], 1e-10);
-        wk[(MW_V + rq * 4 + b * 2 + 0) * W + k] = fl[FPX * W + k] / n;
-        wk[(MW_V + rq * 4 + b * 2 + 1) * W + k] = fl[FPZ * W + k] / n;
+        double vx, vz;
+        velocities(n, fl[FPX * W + k], fl[FPZ * W + k], vx, vz);
+        wk[(MW_V + rq * 4 + b * 2 + 0) * W + k] = vx;
+        wk[(MW_V + rq * 4 + b * 2 + 1) * W + k] = vz;
       }
       __syncthreads();
 

@@ -17,14 +17,15 @@ __device__ __forceinline__ double number(unsigned long long h, int e_lo, int e_n
   return __longlong_as_double((long long)(((h >> 63) << 63) | (e << 52) | mant));
 }
 
-// n >= 0.05 always (the density floor).  kind 0: n near 1, momenta of any
+// n >= 0.05 (the density floor) but in kind 5.  kind 0: n near 1, momenta of any
 // size; 1: n of any size up to 2^100; 2: momenta that put the quotient on or
-// beside a double; 3: n with an all-ones mantissa; 4: special momenta and n.
+// beside a double; 3: n with an all-ones mantissa; 4: special momenta and n;
+// 5: n down to the 1e-10 of the field update.
 __global__ void check(unsigned long long seed, long long count, int kind, unsigned long long* bad, double* first) {
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count; i += stride) {
     const unsigned long long h = mix64(seed ^ mix64((unsigned long long)i)), g = mix64(h + 1), k = mix64(g + 1);
-    double n = fabs(number(h, -4, kind == 1 ? 104 : 8, kind == 3));
+    double n = fabs(number(h, kind == 5 ? -33 : -4, kind == 1 ? 104 : (kind == 5 ? 40 : 8), kind == 3));
     double a = number(g, -1000, 2000, false), b = number(k, -40, 60, false);
     if (kind == 2) {
       a = number(g, -300, 600, false) * n;
@@ -39,7 +40,7 @@ __global__ void check(unsigned long long seed, long long count, int kind, unsign
       b = sp[(i / 12) % 12];
       n = sn[(i / 144) % 4];
     }
-    if (n < 0.05) n = 0.05;
+    n = fmax(n, kind == 5 ? 1e-10 : 0.05);
     double u, v;
     ymkh::velocities(n, a, b, u, v);
     const double wu = a / n, wv = b / n;

@@ -158,7 +158,7 @@ def velocity_checker(cuda, tmp_path_factory):
     return lib
 
 
-@pytest.mark.parametrize("kind", range(5))
+@pytest.mark.parametrize("kind", range(6))
 def test_velocities_are_the_ieee_quotients(velocity_checker, kind):
     bad, first = C.c_ulonglong(), (C.c_double * 2)()
     assert velocity_checker.velocities_check(99 + kind, 1 << 28, kind, C.byref(bad), first) == 0
