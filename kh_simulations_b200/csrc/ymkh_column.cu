@@ -505,10 +505,17 @@ size_t band_coef_smem(int bm) { return sizeof(double2) * (size_t)bm * (2 * BD_CH
 cudaError_t launch_band(const ArrayList& arrs, int narr, const double* W, int ldw, int J, double* C, int nx, int nz,
                         double inv2, cudaStream_t s) {
   const int M = J / 2, nxb = (nx + BD_TX - 1) / BD_TX;
-  // modes per coefficient CTA: as many as leave every SM some CTAs
-  int bm = BC_BM;
-  while (bm > 4 && (long long)((M + bm - 1) / bm) * nxb * narr < 148 * 4) bm /= 2;
-  bm = std::min(bm, M);
+  // Modes per coefficient CTA.  Four CTAs fit an SM and all take equally long,
+  // so while they fill the SMs only a few times, the number whose turns come to
+  // the fewest modes (us at 256 x 512, modes 86..128: 105 against 112 with
+  // halving to four; 512 x 512 320 against 347); beyond, the most that fit,
+  // which read the array least (1024 x 2048 3.66 ms against 3.91).
+  const long long slots = 148 * 4;
+  auto turns = [&](int m) { return ((long long)((M + m - 1) / m) * nxb * narr + slots - 1) / slots; };
+  int bm = std::min(BC_BM, M);
+  if (turns(bm) <= 4)
+    for (int m = bm - 1; m >= 4; --m)
+      if (turns(m) * m < turns(bm) * bm) bm = m;
   band_coef_kernel<<<dim3((M + bm - 1) / bm, nxb, narr), BC_NT, band_coef_smem(bm), s>>>(arrs, W, ldw, M, bm, C, nx, nz, inv2);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
