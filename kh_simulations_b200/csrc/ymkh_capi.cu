@@ -137,6 +137,7 @@ struct ymkh_ctx {
   double* coef = nullptr;    // band coefficients [21][J][nx]
   Tf32BandImages tfb[MAX_BANDS]{};  // TF32 engine: twiddle tile images per band
   Tf32Scratch tfs{};                // TF32 engine: G and C^T tile images
+  double* zmeans = nullptr;         // TF32 engine with suppress_kz0: z-means the first band takes off
   double* epart = nullptr;   // energy partials
   double* hres = nullptr;    // results of the diagnostics: a slot of pinned host memory (on first use)
   double* mcol = nullptr;    // mode amplitude partial sums (allocated on first use)
@@ -220,6 +221,7 @@ void free_bands(ymkh_ctx* c) {
   for (float** q : {&c->tfs.gh, &c->tfs.gl, &c->tfs.ch, &c->tfs.cl})
     if (*q) { cudaFree(*q); *q = nullptr; }
   if (c->coef) { cudaFree(c->coef); c->coef = nullptr; }
+  if (c->zmeans) { cudaFree(c->zmeans); c->zmeans = nullptr; }
   c->nb = 0;
 }
 
@@ -245,6 +247,7 @@ int setup_tf32(ymkh_ctx* c) {
   CK(cudaMalloc(&c->tfs.gl, ng * sizeof(float)), "cudaMalloc TF32 G images");
   CK(cudaMalloc(&c->tfs.ch, nc * sizeof(float)), "cudaMalloc TF32 coefficient images");
   CK(cudaMalloc(&c->tfs.cl, nc * sizeof(float)), "cudaMalloc TF32 coefficient images");
+  if (c->prm.suppress_kz0) CK(cudaMalloc(&c->zmeans, (size_t)12 * c->nx * sizeof(double)), "cudaMalloc z-means");
   return 0;
 }
 
@@ -635,14 +638,16 @@ int post_stages(ymkh_ctx* c, cudaStream_t s) {
   if (c->prm.suppress_kz0) {
     ArrayList zl = filt;  // 12 arrays lose their z-mean, then By1, Ex1, Ez1 are zeroed
     for (int i = 0; i < 3; ++i) zl.p[12 + i] = l21.p[i];
-    CK(launch_zmean(zl, 12, 3, c->nx, c->nz, s), "zmean");
+    CK(launch_zmean(zl, 12, 3, c->nx, c->nz, c->zmeans, s), "zmean");
     g_launches++;
   }
   mark(c, ST_BANDS, s);
   const double inv2 = (double)(2.0f / (float)c->nz);
   for (int b = 0; b < c->nb; ++b) {
     if (c->prm.filter_engine == YMKH_FILTER_TF32X3) {
-      CK(launch_band_tf32(filt, 21 - skip, c->tfb[b], c->tfs, c->nx, c->nz, 2.0f / (float)c->nz, c->derr, s),
+      // the first band also takes off the z-means (filt's first 12 arrays)
+      CK(launch_band_tf32(filt, 21 - skip, c->tfb[b], c->tfs, c->nx, c->nz, 2.0f / (float)c->nz, c->zmeans,
+                          c->zmeans && b == 0 ? 12 : 0, c->derr, s),
          "band filter (TF32 tensor cores)");
       g_launches += 3;
     } else {

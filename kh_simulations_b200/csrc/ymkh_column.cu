@@ -88,7 +88,8 @@ cudaError_t launch_sponge_xicut(const ArrayList& a12, const StepParams& p, int c
 // halving tree (YM_Physics.cu:301-308) so the mean is bit-identical.
 constexpr int ZM_CX = 4;
 constexpr size_t kColumnSmemMax = 200 * 1024;  // shared memory of the staged-column kernels
-__global__ void zmean_kernel(const __grid_constant__ ArrayList arrs, int nx, int nz, int nmean) {
+__global__ void zmean_kernel(const __grid_constant__ ArrayList arrs, int nx, int nz, int nmean,
+                             double* __restrict__ means) {
   extern __shared__ double sm[];  // [nz][ZM_CX]
   const int x0 = blockIdx.x * ZM_CX;
   double* g = arrs.p[blockIdx.y];
@@ -109,6 +110,10 @@ __global__ void zmean_kernel(const __grid_constant__ ArrayList arrs, int nx, int
     __syncthreads();
   }
   const double inv = 1.0 / (double)nz;
+  if (means) {
+    if (threadIdx.x < ZM_CX && x0 + threadIdx.x < nx) means[(size_t)blockIdx.y * nx + x0 + threadIdx.x] = sm[threadIdx.x] * inv;
+    return;
+  }
   for (int i = threadIdx.x; i < nz * ZM_CX; i += blockDim.x) {
     const int z = i / ZM_CX, c = i - z * ZM_CX;
     if (x0 + c < nx) {
@@ -129,7 +134,8 @@ __global__ void zmean_kernel(const __grid_constant__ ArrayList arrs, int nx, int
 // halving tree's, bit for bit; the columns are then re-read (mostly from L2)
 // and the mean subtracted.
 template <int LOGM>
-__global__ void __launch_bounds__(1024) zmean_p2_kernel(const __grid_constant__ ArrayList arrs, int nx, int nmean) {
+__global__ void __launch_bounds__(1024) zmean_p2_kernel(const __grid_constant__ ArrayList arrs, int nx, int nmean,
+                                                        double* __restrict__ means) {
   constexpr int M = 1 << LOGM;
   __shared__ double part[32][33];
   __shared__ double mean[32];
@@ -168,6 +174,10 @@ __global__ void __launch_bounds__(1024) zmean_p2_kernel(const __grid_constant__ 
     if (lane == 0) mean[l] = v * (1.0 / (double)(32 * M));
   }
   __syncthreads();
+  if (means) {
+    if (in && l == 0) means[(size_t)blockIdx.y * nx + x] = mean[lane];
+    return;
+  }
   if (in) {
     const double mu = mean[lane];
 #pragma unroll 8
@@ -178,23 +188,23 @@ __global__ void __launch_bounds__(1024) zmean_p2_kernel(const __grid_constant__ 
   }
 }
 
-cudaError_t launch_zmean(const ArrayList& arrs, int nmean, int nzero, int nx, int nz, cudaStream_t s) {
+cudaError_t launch_zmean(const ArrayList& arrs, int nmean, int nzero, int nx, int nz, double* means, cudaStream_t s) {
   const int narr = nmean + nzero;
   const dim3 g32((nx + 31) / 32, narr);
   switch (nz) {
-    case 128: zmean_p2_kernel<2><<<g32, 1024, 0, s>>>(arrs, nx, nmean); return cudaGetLastError();
-    case 256: zmean_p2_kernel<3><<<g32, 1024, 0, s>>>(arrs, nx, nmean); return cudaGetLastError();
-    case 512: zmean_p2_kernel<4><<<g32, 1024, 0, s>>>(arrs, nx, nmean); return cudaGetLastError();
-    case 1024: zmean_p2_kernel<5><<<g32, 1024, 0, s>>>(arrs, nx, nmean); return cudaGetLastError();
-    case 2048: zmean_p2_kernel<6><<<g32, 1024, 0, s>>>(arrs, nx, nmean); return cudaGetLastError();
-    case 4096: zmean_p2_kernel<7><<<g32, 1024, 0, s>>>(arrs, nx, nmean); return cudaGetLastError();
-    case 8192: zmean_p2_kernel<8><<<g32, 1024, 0, s>>>(arrs, nx, nmean); return cudaGetLastError();
+    case 128: zmean_p2_kernel<2><<<g32, 1024, 0, s>>>(arrs, nx, nmean, means); return cudaGetLastError();
+    case 256: zmean_p2_kernel<3><<<g32, 1024, 0, s>>>(arrs, nx, nmean, means); return cudaGetLastError();
+    case 512: zmean_p2_kernel<4><<<g32, 1024, 0, s>>>(arrs, nx, nmean, means); return cudaGetLastError();
+    case 1024: zmean_p2_kernel<5><<<g32, 1024, 0, s>>>(arrs, nx, nmean, means); return cudaGetLastError();
+    case 2048: zmean_p2_kernel<6><<<g32, 1024, 0, s>>>(arrs, nx, nmean, means); return cudaGetLastError();
+    case 4096: zmean_p2_kernel<7><<<g32, 1024, 0, s>>>(arrs, nx, nmean, means); return cudaGetLastError();
+    case 8192: zmean_p2_kernel<8><<<g32, 1024, 0, s>>>(arrs, nx, nmean, means); return cudaGetLastError();
     default: break;
   }
   const size_t smem = (size_t)nz * ZM_CX * sizeof(double);
   if (smem > kColumnSmemMax) return cudaErrorInvalidValue;  // NZ > 6400 without a coalesced form
   dim3 grid((nx + ZM_CX - 1) / ZM_CX, narr);
-  zmean_kernel<<<grid, 256, smem, s>>>(arrs, nx, nz, nmean);
+  zmean_kernel<<<grid, 256, smem, s>>>(arrs, nx, nz, nmean, means);
   return cudaGetLastError();
 }
 

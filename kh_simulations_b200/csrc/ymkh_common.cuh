@@ -225,8 +225,9 @@ cudaError_t prepare_maxwell();
 int maxwell_ctas_per_sm();
 cudaError_t launch_sponge_xicut(const ArrayList& a12, const StepParams& p, int cut, cudaStream_t s);
 cudaError_t prepare_column(int nz);
-// The z-mean of arrs[0, nmean) removed and arrs[nmean, nmean + nzero) zeroed, in one launch.
-cudaError_t launch_zmean(const ArrayList& arrs, int nmean, int nzero, int nx, int nz, cudaStream_t s);
+// The z-mean of arrs[0, nmean) removed and arrs[nmean, nmean + nzero) zeroed, in
+// one launch.  With means, [nmean][nx], they are written there, not removed.
+cudaError_t launch_zmean(const ArrayList& arrs, int nmean, int nzero, int nx, int nz, double* means, cudaStream_t s);
 cudaError_t launch_hyperdiff(const ArrayList& a12, int nx, int nz, double mu, cudaStream_t s);
 cudaError_t launch_band(const ArrayList& arrs, int narr, const double* W, int ldw, int J, double* C, int nx, int nz,
                         double inv2, cudaStream_t s);
@@ -270,7 +271,7 @@ size_t tf32_tile_floats();
 cudaError_t prepare_tf32();
 cudaError_t launch_tf32_w_images(const double* W, int ldw, int J, int nz, const Tf32BandImages& b, cudaStream_t s);
 cudaError_t launch_band_tf32(const ArrayList& arrs, int narr, const Tf32BandImages& b, const Tf32Scratch& w, int nx,
-                             int nz, float inv2, unsigned* err, cudaStream_t s);
+                             int nz, float inv2, const double* means, int nmean, unsigned* err, cudaStream_t s);
 int capi_error(int code, const char* msg);
 void capi_count_launches(int n);
 

@@ -135,6 +135,11 @@ __global__ void w_image_kernel(const double* __restrict__ W, int ldw, int J, int
   a2l[t2] = lo;
 }
 
+// With suppress_kz0 the z-means of the first arrays arrive as one value a
+// column: this kernel takes them off on its way to the images and GEMM 2's
+// epilogue where it updates G, so the z-mean stage only has to read (bit for
+// bit the subtraction it would have stored).
+//
 // G_k[z, x] (FP64) -> B image of GEMM 1, tile (nt, kt) of array k: rows x,
 // k = z.  Thread (x, z-quad): four loads along z (each coalesced across the
 // warp's consecutive x), split, and one 16-byte store per hi/lo chunk into
@@ -142,20 +147,21 @@ __global__ void w_image_kernel(const double* __restrict__ W, int ldw, int J, int
 // conflict-free); the tile is then written out linearly.
 __global__ void __launch_bounds__(256)
     g_image_kernel(const __grid_constant__ ArrayList arrs, int nx, int nz, int NT, int KT, float* __restrict__ gh,
-                   float* __restrict__ gl) {
+                   float* __restrict__ gl, const double* __restrict__ means, int nmean) {
   __shared__ __align__(16) float sh[TT_FLOATS];
   __shared__ __align__(16) float sl[TT_FLOATS];
   const int nt = blockIdx.x, kt = blockIdx.y, k = blockIdx.z;
   const double* G = arrs.p[k];
   const int xx = threadIdx.x % TT_IMG_N, qh = threadIdx.x / TT_IMG_N;  // 2 halves of the 8 z-quads
   const int x = nt * TT_IMG_N + xx;
+  const double mean = (k < nmean && x < nx) ? means[(size_t)k * nx + x] : 0.0;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const int q = qh * 4 + j;  // 16-byte chunk (4 consecutive z) of the tile row
     const int z = kt * TT_K + 4 * q;
     double g[4];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) g[c] = (x < nx && z + c < nz) ? G[(size_t)(z + c) * nx + x] : 0.0;
+    for (int c = 0; c < 4; ++c) g[c] = (x < nx && z + c < nz) ? G[(size_t)(z + c) * nx + x] - mean : 0.0;
     float4 h, l;
     split_f64(g[0], h.x, l.x);
     split_f64(g[1], h.y, l.y);
@@ -207,8 +213,10 @@ struct Tf32GemmArgs {
   float* c_lo;
   int KT2;
   float scale;
-  // EPI_APPLY: G_k[z, x] -= D[x, z]
+  // EPI_APPLY: G_k[z, x] = (G_k[z, x] - mean_k[x]) - D[x, z]
   ArrayList arrs;
+  const double* means;  // z-means still to be taken off the first nmean arrays
+  int nmean;
   int nx;
   int nz;
   unsigned* err;
@@ -394,16 +402,17 @@ __global__ void __launch_bounds__(WS_THREADS, 1) tf32x3_gemm_ws(const __grid_con
           if (x < g.nx && z0 < g.nz) {
             double* const G = g.arrs.p[k] + (size_t)z0 * g.nx + x;
             const size_t ld = (size_t)g.nx;
+            const double mean = k < g.nmean ? g.means[(size_t)k * ld + x] : 0.0;  // (v - 0.0 is v)
             if (z0 + 32 <= g.nz) {
               double gv[32];
 #pragma unroll
               for (int c = 0; c < 32; ++c) gv[c] = G[(size_t)c * ld];
 #pragma unroll
-              for (int c = 0; c < 32; ++c) G[(size_t)c * ld] = gv[c] - (double)__uint_as_float(v[c]);
+              for (int c = 0; c < 32; ++c) G[(size_t)c * ld] = (gv[c] - mean) - (double)__uint_as_float(v[c]);
             } else {
 #pragma unroll
               for (int c = 0; c < 32; ++c)
-                if (z0 + c < g.nz) G[(size_t)c * ld] = G[(size_t)c * ld] - (double)__uint_as_float(v[c]);
+                if (z0 + c < g.nz) G[(size_t)c * ld] = (G[(size_t)c * ld] - mean) - (double)__uint_as_float(v[c]);
             }
           }
         }
@@ -474,11 +483,11 @@ cudaError_t launch_tf32_w_images(const double* W, int ldw, int J, int nz, const 
 }
 
 cudaError_t launch_band_tf32(const ArrayList& arrs, int narr, const Tf32BandImages& b, const Tf32Scratch& w, int nx,
-                             int nz, float inv2, unsigned* err, cudaStream_t s) {
+                             int nz, float inv2, const double* means, int nmean, unsigned* err, cudaStream_t s) {
   if (narr < 1) return cudaErrorInvalidValue;
   const int Zp = tf32_zpad(nz);
   const int NT = tf32_ntiles(nx), KT1 = Zp / TT_K, MT1 = b.Jp / TT_M, KT2 = b.Jp / TT_K, MT2 = Zp / TT_M;
-  g_image_kernel<<<dim3(NT, KT1, narr), 256, 0, s>>>(arrs, nx, nz, NT, KT1, w.gh, w.gl);
+  g_image_kernel<<<dim3(NT, KT1, narr), 256, 0, s>>>(arrs, nx, nz, NT, KT1, w.gh, w.gl, means, nmean);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   int dev = 0, sms = 148;
@@ -499,6 +508,8 @@ cudaError_t launch_band_tf32(const ArrayList& arrs, int narr, const Tf32BandImag
   g1.KT2 = KT2;
   g1.scale = inv2;
   g1.arrs = arrs;
+  g1.means = means;
+  g1.nmean = nmean;
   g1.nx = nx;
   g1.nz = nz;
   g1.err = err;

@@ -117,3 +117,35 @@ def test_batch_follows_a_members_new_parameters(cuda):
     assert np.array_equal(runs[1].state_numpy(), ref.state_numpy())
     assert not np.array_equal(runs[0].state_numpy(), ref.state_numpy())
     batch.close()
+
+
+@pytest.mark.parametrize("nz,nx", [(64, 130), (128, 96), (1024, 40)])
+@pytest.mark.parametrize("bands", ["kz_keep_max = {third}\n", "kz_bands = 3-9,12-20\n"])
+def test_zmean_taken_off_by_the_tf32_filter(cuda, nz, nx, bands):
+    """suppress_kz0 with the TF32 engine, whose first band takes the z-means
+    off, bit for bit the z-mean stage followed by the filter.  On a fluid at
+    rest without fields, sweeps and field update leave Az2 and Az3 as they are,
+    so the two stages can be had one after the other in two runs."""
+    from kh_simulations_b200.run import KHRun
+
+    tf32 = "filter_engine = tf32x3\n" + bands
+    runs = [KHRun(_config(s, nz, nx)) for s in (KZ0 + tf32, KZ0, tf32)]
+    both, mean, band = runs
+    st = np.zeros((24, nz, nx))
+    rng = np.random.default_rng(nz + nx)
+    st[10:12] = rng.normal(0.3, 1.0, size=(2, nz, nx))
+    st[[12, 18]] = 1.0
+    st[15], st[21] = 1.0, -1.0
+    both.set_state(st)
+    mean.set_state(st)
+    both.step(1)
+    mean.step(1)
+    s = mean.state_numpy()
+    assert not np.array_equal(s[10:12], st[10:12]) and np.array_equal(s[12:], st[12:])
+    band.set_state(s)
+    band.step(1)
+    a, b = both.state_numpy(), band.state_numpy()
+    assert not np.array_equal(a[10:12], s[10:12])
+    assert np.array_equal(a[10:12].view(np.uint64), b[10:12].view(np.uint64))
+    for r in runs:
+        r.close()
