@@ -2,12 +2,14 @@
 // lifetime, state binding, the step sequence and the diagnostics.
 //
 // The step keeps the reference's stage order (ymgpu2d/main_ym.cu:324-455):
-//   FCT x+z sweeps of both beams, density floor   -> fct_fused_kernel
+//   FCT x+z sweeps of both beams, density floor   -> fct_strip_kernel / fct_fused_kernel
 //   currents, Ampère, potential, Faraday          -> maxwell_fused_kernel
 //   sponge, xi_cut                                -> sponge_xicut_kernel
 //   z-mean removal and colour-1 EM zeroing        -> zmean_p2_kernel / zmean_kernel
 //   DFT kz bands on the 21 filtered arrays        -> band_coef / band_apply
 //   z-hyperdiffusion                              -> hyperdiff_kernel
+// (the stages from the sponge on in one launch of column_kernel, where
+// col_fused_alone and the batch say so).
 // The sources of stage 7 are recomputed inside the next FCT launch.
 //
 // The stencil kernels read start-of-step values of neighbouring tiles, so
@@ -673,7 +675,7 @@ bool has_column_stages(const ymkh_ctx* c) {
 // One reference iteration from buffer c->cur into buffer 1 - c->cur.
 int step_once(ymkh_ctx* c, cudaStream_t s) {
   { int rc = flush_desc(c, s); if (rc) return rc; }
-  RunTable T{c->dev->desc + c->cur, 1, c->fct_items, c->mx_items, c->derr, c->fx_items, c->fz_items, 1, c->dev->fct_first};
+  RunTable T{c->dev->desc + c->cur, 1, c->fct_items, c->mx_items, c->derr, c->fx_items, c->fz_items, c->dev->fct_first};
   mark(c, ST_FCT, s);
   {
     NvtxRange r("ymkh fct");
@@ -1277,7 +1279,7 @@ int batch_build(ymkh_batch* b, cudaStream_t s) {
 int batch_step_once(ymkh_batch* b, cudaStream_t s) {
   const int n = (int)b->runs.size();
   if (!n) return 0;
-  RunTable T{b->ddesc + (size_t)b->parity * b->cap, n, b->fct_items, b->mx_items, b->derr, b->fx_items, b->fz_items, 1, b->dfirst};
+  RunTable T{b->ddesc + (size_t)b->parity * b->cap, n, b->fct_items, b->mx_items, b->derr, b->fx_items, b->fz_items, b->dfirst};
   if (b->fct_mode == YMKH_FCT_SPLIT)
     CK(launch_fct_split_table(T, b->fx_grid, b->fz_grid, s), "fct_x/fct_z kernels (batch)");
   else

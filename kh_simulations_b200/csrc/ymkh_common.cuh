@@ -147,10 +147,6 @@ __device__ __forceinline__ int xmap(int x, int nx, int periodic) {
   return x < 0 ? 0 : (x >= nx ? nx - 1 : x);
 }
 __device__ __forceinline__ int zclamp(int z, int nz) { return z < 0 ? 0 : (z >= nz ? nz - 1 : z); }
-__device__ __forceinline__ int zwrap(int z, int nz) {
-  z %= nz;
-  return z < 0 ? z + nz : z;
-}
 
 __device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
   unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -361,10 +357,11 @@ __device__ __forceinline__ void bulk_row_periodic(double* dst, const double* row
 namespace ymkh {
 
 // How a fused kernel stages its rows (RunDesc::fct_bulk / mx_bulk).
-// Measured at 4096 x 8192 (FCT / Maxwell per step): TMA bulk rows issued
-// by warp 0 alone 9.0 / 4.5 ms, 16-byte cp.async by every thread 7.8 / 4.1
-// ms, bulk rows spread one per thread over all warps 7.3 / 3.9 ms (the form
-// kept).
+// Of the row copies, one per thread spread over the warps is the fastest form
+// (FCT / Maxwell of an early build at 4096 x 8192: 7.3 / 3.9 ms, against 7.8 /
+// 4.1 for 16-byte cp.async by every thread and 9.0 / 4.5 for TMA rows from one
+// warp).  Boxes take their place where the arrays allow it: one thread's three
+// or two requests a row instead of 33 or 24 (Maxwell 1.91 -> 1.82 ms).
 enum RowLoad : int {
   LOAD_ELEM = 0,    // per-element 8-byte cp.async through an x index table (walls, odd nx)
   LOAD_BULK_ALL = 3, // TMA bulk row copies, one per thread spread over all warps
@@ -397,7 +394,6 @@ struct RunTable {
   int fct_items, mx_items;
   unsigned* err;  // device error word of the bounded in-kernel waits
   int fx_items, fz_items;
-  int fct_contig;  // fused FCT: 1 = contiguous item blocks per CTA, 0 = round-robin
   const int* fct_first;  // 128-wide FCT: CTA b takes the items [fct_first[b], fct_first[b + 1])
 };
 

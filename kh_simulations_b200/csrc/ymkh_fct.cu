@@ -11,9 +11,13 @@
 // kernel_ym_precession, YM_Fluid.cu:32-108) are recomputed here from the
 // start-of-step state, which is what they are a function of.
 //
-// Layout: work items are (x-strip, z-segment) pairs; for a lone run each
-// persistent CTA takes a contiguous block of them and runs each strip's part
-// as one piece, for batches the CTAs take them round-robin.  A strip emits TB-6 columns; thread t of a beam owns
+// Two forms: fct_strip_kernel (128-wide strips, one warp per variable, further
+// down with its own comment) for all but the smallest grids and for batches,
+// and fct_fused_kernel<32 | 64>, described here.
+//
+// Layout: work items are (x-strip, z-segment) pairs; each persistent CTA takes
+// a contiguous block of them and runs each strip's part as one piece.  A strip
+// emits TB-6 columns; thread t of a beam owns
 // stage position t+1 (shear index x0-3+t), and every x-sweep phase is at
 // most one position or interface per thread: interface quantities (eps, nu,
 // mu, low-order fluxes) are formed once per interface.  Threads [0,TB)
@@ -142,18 +146,14 @@ __global__ void __launch_bounds__(4 * TB, 2)
   unsigned issued = 0, consumed = 0;  // rows issued / consumed by this CTA (all items)
   unsigned phase_bits = 0;            // per-stage mbarrier phase of the bulk path
 
-  // Lone run (T.fct_contig): each CTA takes one contiguous block of the
-  // flattened items.  Within a run the items are strip-major (a strip's
-  // z-segments consecutive), and consecutive segments of one strip form one
-  // piece: the z pipeline warms up (6 rows) once per piece instead of once
-  // per segment, and the blocks differ by at most one segment.  Batches
-  // take segment-major items round-robin, so the CTAs running at once work
-  // on neighbouring strips of the same rows and share halos through L2
-  // (3.5% faster on an uneven 64-run sweep).
-  const bool contig = T.fct_contig != 0;
-  const int per = contig ? (T.fct_items + (int)gridDim.x - 1) / (int)gridDim.x : 0;
-  const int i_beg = contig ? (int)blockIdx.x * per : (int)blockIdx.x;
-  const int i_end = contig ? min(T.fct_items, i_beg + per) : T.fct_items;
+  // Each CTA takes one contiguous block of the flattened items.  Within a run
+  // the items are strip-major (a strip's z-segments consecutive), and
+  // consecutive segments of one strip form one piece: the z pipeline warms up
+  // (6 rows) once per piece instead of once per segment, and the blocks differ
+  // by at most one segment.
+  const int per = (T.fct_items + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int i_beg = (int)blockIdx.x * per;
+  const int i_end = min(T.fct_items, i_beg + per);
   int next = i_beg;
   for (int item = i_beg; item < i_end; item = next) {
     __syncthreads();  // previous piece fully consumed
@@ -170,19 +170,11 @@ __global__ void __launch_bounds__(4 * TB, 2)
     const double dtdz = p.dt / p.dz;
     const int nseg = (nz + rd.fct_seg - 1) / rd.fct_seg;
     const int local = item - rd.fct_item0;
-    int strip, zs, ze;
-    if (contig) {
-      strip = local / nseg;
-      const int seg0 = local - strip * nseg;
-      next = min(i_end, rd.fct_item0 + (strip + 1) * nseg);  // past this piece's last segment
-      zs = seg0 * rd.fct_seg;
-      ze = min(nz, (seg0 + (next - item)) * rd.fct_seg);
-    } else {
-      strip = local % rd.fct_nstrips;
-      zs = (local / rd.fct_nstrips) * rd.fct_seg;
-      ze = min(nz, zs + rd.fct_seg);
-      next = item + (int)gridDim.x;
-    }
+    const int strip = local / nseg;
+    const int seg0 = local - strip * nseg;
+    next = min(i_end, rd.fct_item0 + (strip + 1) * nseg);  // past this piece's last segment
+    const int zs = seg0 * rd.fct_seg;
+    const int ze = min(nz, (seg0 + (next - item)) * rd.fct_seg);
     const int x0 = strip * TO;
 
     if (!bulk)
@@ -515,12 +507,15 @@ __global__ void __launch_bounds__(4 * TB, 2)
 //   through the NaN-exact form.
 // - The sweep warps hold 72 registers of z history: setmaxnreg gives them 136
 //   and the coefficient warps 104 of the 512 x 128 at launch.
-// Measured (FCT, one step, against the 128-wide fct_fused_kernel): 3.42 ms
-// against 5.17 at 4096 x 8192, 251 us against 366 at 1024 x 2048.  Tried and
-// slower: the z history rotated through names by unrolling the row loop two or
-// three times (no register moves, but spills and a loop past the instruction
-// cache: 3.6 and 5.3 ms), separate fast and slow row loops, a CTA barrier per
-// row in place of the mbarriers, divisions in place of `velocities` (4% more).
+// Measured (FCT, one step, against the 128-wide fct_fused_kernel that it took
+// the place of): 3.12 ms against 5.17 at 4096 x 8192, 227 us against 366 at
+// 1024 x 2048, 56 against 73 at 256 x 768; of that, blocks cut by cost
+// (3.42 -> 3.12 ms together with boxes for the edge strips).  Tried and slower
+// (ms against the 3.4 to 3.9 of the kernel at the time): the z history rotated
+// through names by unrolling the row loop two or three times (no register
+// moves, but spills and a loop past the instruction cache: 3.6 and 5.3),
+// separate fast and slow row loops, a CTA barrier per row in place of the
+// mbarriers, divisions in place of `velocities` (4% more).
 
 namespace {
 
@@ -1066,10 +1061,8 @@ static cudaError_t prepare_fct_t() {
                               (int)fct_smem_bytes<TB>(NST));
 }
 
-// Stage ring depth (rows in flight = NST - 1).  Measured on B200 with
-// 128-wide strips, step ms at 4096 x 8192 / 1024 x 2048: 7.38 / 0.522 with
-// 2 stages, 7.18 / 0.505 with 3, 7.06 / 0.497 with 4 (206 KB of shared
-// memory; 5 stages do not fit).  64-wide strips run 2 CTAs of 4 stages per SM.
+// Stage ring depth of fct_fused_kernel (rows in flight = NST - 1): with four
+// stages two CTAs of 64-wide strips fit an SM's shared memory, with five one.
 template <int TB>
 constexpr int fct_nst() {
   return 4;
@@ -1087,7 +1080,8 @@ int fct_bulk_ok(const StepParams& p, int tb) {
 // The kernel reads start-of-step values across strip and segment halos while
 // other CTAs write theirs, so each run's fluid goes to its second buffer
 // (`out`); fields are only read.  grid_ctas persistent CTAs take contiguous
-// blocks of the flattened (run, strip, segment) items.
+// blocks of the flattened (run, strip, segment) items; the 128-wide form's
+// blocks are T.fct_first's.
 cudaError_t launch_fct_table(const RunTable& T, int tb, int grid_ctas, cudaStream_t s) {
   const int grid = std::max(1, std::min(T.fct_items, grid_ctas));
   switch (tb) {
