@@ -156,7 +156,7 @@ struct ymkh_ctx {
     TensorMap maps[2 * kMaps];     // kMaps of buffer 0, then of buffer 1
     RunDesc desc[2];               // run descriptors for start buffer 0 and 1
     ColDesc col[2];                // column stages writing buffer 0 and buffer 1
-    int fct_first[kMaxFctCtas + 1];  // items of the 128-wide FCT's CTAs
+    int fct_first[kMaxFctCtas + 1];  // items of the fused FCT's CTAs
   };
   Tables host{};              // host copy
   Tables* dev = nullptr;      // device copy
@@ -506,47 +506,60 @@ bool col_fused_alone(const ymkh_ctx* c) {
   return stages >= 2 || (c->nb && c->nz <= 128);
 }
 
-// How the 128-wide FCT's items (strip-major segments) are cut into one
-// contiguous block per CTA.  The launch lasts as long as its slowest CTA, so
-// the blocks are equal in cost, not in rows: in units of a fifth of an inner
+// How the fused FCT's items (strip-major segments) are cut into one contiguous
+// block per CTA.  The launch lasts as long as its slowest CTA, so the cut is
+// the one whose costliest block is cheapest: in units of a fifth of an inner
 // strip's row, a row of a strip whose window wraps takes 6 (its wrapped columns
 // are put in place separately: 480 against 400 thousand cycles for 131 rows),
-// and entering a strip kFctEntry more (its pipeline's fill).  With few rows per
-// CTA the cut is by rows: there a whole row decides.  FCT of one step, against
-// equal rows: 3.42 -> 3.12 ms at 4096 x 8192, 252 -> 227 us at 1024 x 2048
-// (entry 0, 20, 60: 236, 229, 227; edge row 7: 230).
+// and every strip that a block enters kFctEntry more (six rows of warm-up and
+// the pipeline's fill).  So on a large grid the blocks even out (against equal
+// rows 3.42 -> 3.12 ms at 4096 x 8192, 252 -> 227 us at 1024 x 2048), and on a
+// small one none runs on into a second strip for a few rows (FCT us, against
+// equal rows there: 128 x 256 38 -> 27, 256 x 512 48 -> 37, 256 x 768 56 -> 42,
+// walls of 64-wide strips 243 x 371 71 -> 61; entry 25: 45 at 256 x 768, 60 as
+// 40).
 struct StripRun {
   int nstrips, nseg, seg;
   bool box;
 };
-constexpr int kFctEntry = 40, kFctEdgeRow = 6, kFctInnerRow = 5, kFctEvenBelow = 16;
-void cut_fct(const std::vector<StripRun>& runs, int grid, int* first) {
-  long long items = 0, rows = 0, cost = 0;
-  auto row_cost = [](const StripRun& r, int s) { return r.box && (s == 0 || s == r.nstrips - 1) ? kFctEdgeRow : kFctInnerRow; };
-  for (const StripRun& r : runs) {
-    items += (long long)r.nstrips * r.nseg;
-    rows += (long long)r.nstrips * r.nseg * r.seg;
-    for (int s = 0; s < r.nstrips; ++s) cost += kFctEntry + (long long)r.nseg * r.seg * row_cost(r, s);
-  }
-  first[0] = 0;
-  if (rows < (long long)kFctEvenBelow * grid) {
-    const long long per = (items + grid - 1) / std::max(grid, 1);
-    for (int b = 1; b <= grid; ++b) first[b] = (int)std::min(items, b * per);
-    return;
-  }
-  int b = 1;
-  long long at = 0, item = 0;  // cost and items ahead of the strip
+constexpr int kFctEntry = 40, kFctEdgeRow = 6, kFctInnerRow = 5;
+// Cuts the items into blocks of cost `most` or less; returns how many that
+// takes, and with `first` writes where each starts.
+int cut_fct_at(const std::vector<StripRun>& runs, long long most, int* first) {
+  int n = 0, item = 0;
+  long long left = 0;
   for (const StripRun& r : runs)
     for (int s = 0; s < r.nstrips; ++s) {
-      const long long unit = (long long)r.seg * row_cost(r, s), end = at + kFctEntry + r.nseg * unit;
-      for (; b < grid && cost * b / grid < end; ++b) {
-        const long long into = cost * b / grid - at - kFctEntry;
-        first[b] = (int)(item + (into <= 0 ? 0 : std::min<long long>(r.nseg, (into + unit / 2) / unit)));
+      const long long unit = (long long)r.seg * (r.box && (s == 0 || s == r.nstrips - 1) ? kFctEdgeRow : kFctInnerRow);
+      for (int rem = r.nseg; rem > 0;) {
+        if (left < kFctEntry + unit) {
+          if (first) first[n] = item;
+          ++n;
+          left = most;
+        }
+        const int take = (int)std::min<long long>(rem, std::max<long long>(1, (left - kFctEntry) / unit));
+        left -= kFctEntry + take * unit;
+        rem -= take;
+        item += take;
       }
-      at = end;
-      item += r.nseg;
     }
-  for (; b <= grid; ++b) first[b] = (int)items;
+  return n;
+}
+void cut_fct(const std::vector<StripRun>& runs, int grid, int* first) {
+  long long lo = 1, hi = 0;  // the cheapest `most` lies in [lo, hi]
+  int items = 0;
+  for (const StripRun& r : runs) {
+    items += r.nstrips * r.nseg;
+    hi += r.nstrips * (kFctEntry + (long long)r.nseg * r.seg * kFctEdgeRow);
+    lo = std::max(lo, kFctEntry + (long long)r.seg * kFctEdgeRow);
+  }
+  while (lo < hi) {
+    const long long mid = lo + (hi - lo) / 2;
+    if (cut_fct_at(runs, mid, nullptr) <= grid) hi = mid;
+    else lo = mid + 1;
+  }
+  const int n = cut_fct_at(runs, lo, first);
+  for (int b = n; b <= grid; ++b) first[b] = items;
 }
 StripRun strip_run(const RunDesc& d, int nz) {
   return {d.fct_nstrips, (nz + d.fct_seg - 1) / d.fct_seg, d.fct_seg, d.fct_bulk == LOAD_BOX};
@@ -568,7 +581,7 @@ int upload_desc(ymkh_ctx* c) {
   h[1] = make_desc(c, 1, c->fct_tx, 0, 0);
   for (int i = 0; i < 2; ++i) h[i].fx_item0 = h[i].fz_item0 = 0;
   c->fct_items = items_fct(h[0], c->nz);
-  if (c->fct_tx == 128) cut_fct({strip_run(h[0], c->nz)}, fct_ctas(c->fct_items, c->fct_grid), c->host.fct_first);
+  cut_fct({strip_run(h[0], c->nz)}, fct_ctas(c->fct_items, c->fct_grid), c->host.fct_first);
   c->mx_items = items_mx(h[0], c->nz);
   c->fx_items = items_fx(h[0], c->nz);
   c->fz_items = items_fz(h[0], c->nz);
@@ -1144,7 +1157,7 @@ struct ymkh_batch {
   // members whose column stages run fused, grouped by NZ (one launch a group)
   struct ColGroup { int nz, first, n, items; size_t smem; };
   ColDesc* dcol = nullptr;   // [2][cap]
-  int* dfirst = nullptr;     // items of the 128-wide FCT's CTAs
+  int* dfirst = nullptr;     // items of the fused FCT's CTAs
   std::vector<ColGroup> col;
   std::vector<char> col_member;    // whether the member is in one of the groups
   std::vector<unsigned> versions;  // of the members' descriptors when the tables were built

@@ -394,7 +394,7 @@ struct RunTable {
   int fct_items, mx_items;
   unsigned* err;  // device error word of the bounded in-kernel waits
   int fx_items, fz_items;
-  const int* fct_first;  // 128-wide FCT: CTA b takes the items [fct_first[b], fct_first[b + 1])
+  const int* fct_first;  // fused FCT: CTA b takes the items [fct_first[b], fct_first[b + 1])
 };
 
 // Run owning item g of the split FCT's x pass (which = 0) or z pass (1).

@@ -149,11 +149,9 @@ __global__ void __launch_bounds__(4 * TB, 2)
   // Each CTA takes one contiguous block of the flattened items.  Within a run
   // the items are strip-major (a strip's z-segments consecutive), and
   // consecutive segments of one strip form one piece: the z pipeline warms up
-  // (6 rows) once per piece instead of once per segment, and the blocks differ
-  // by at most one segment.
-  const int per = (T.fct_items + (int)gridDim.x - 1) / (int)gridDim.x;
-  const int i_beg = (int)blockIdx.x * per;
-  const int i_end = min(T.fct_items, i_beg + per);
+  // (6 rows) once per piece instead of once per segment.  The host cuts the
+  // blocks by cost.
+  const int i_beg = T.fct_first[blockIdx.x], i_end = T.fct_first[blockIdx.x + 1];
   int next = i_beg;
   for (int item = i_beg; item < i_end; item = next) {
     __syncthreads();  // previous piece fully consumed
@@ -491,7 +489,7 @@ __global__ void __launch_bounds__(4 * TB, 2)
 // at four warps a scheduler.  fct_fused_kernel issues 114 warp instructions a
 // cell: every phase of the x sweep goes through shared memory and a barrier,
 // each thread group forms its own velocities, and each row costs 33 row
-// copies.  Here a row costs 78:
+// copies.  Here it is 73:
 // - Twelve sweep warps take one variable of one beam each.  A lane owns four
 //   neighbouring columns, so most neighbours are its own registers and the
 //   rest come by shuffles; there is no barrier between the phases, and the
@@ -509,7 +507,7 @@ __global__ void __launch_bounds__(4 * TB, 2)
 //   and the coefficient warps 104 of the 512 x 128 at launch.
 // Measured (FCT, one step, against the 128-wide fct_fused_kernel that it took
 // the place of): 3.12 ms against 5.17 at 4096 x 8192, 227 us against 366 at
-// 1024 x 2048, 56 against 73 at 256 x 768; of that, blocks cut by cost
+// 1024 x 2048, 42 against 73 at 256 x 768; of that, blocks cut by cost
 // (3.42 -> 3.12 ms together with boxes for the edge strips).  Tried and slower
 // (ms against the 3.4 to 3.9 of the kernel at the time): the z history rotated
 // through names by unrolling the row loop two or three times (no register
@@ -1080,8 +1078,7 @@ int fct_bulk_ok(const StepParams& p, int tb) {
 // The kernel reads start-of-step values across strip and segment halos while
 // other CTAs write theirs, so each run's fluid goes to its second buffer
 // (`out`); fields are only read.  grid_ctas persistent CTAs take contiguous
-// blocks of the flattened (run, strip, segment) items; the 128-wide form's
-// blocks are T.fct_first's.
+// blocks of the flattened (run, strip, segment) items, T.fct_first's.
 cudaError_t launch_fct_table(const RunTable& T, int tb, int grid_ctas, cudaStream_t s) {
   const int grid = std::max(1, std::min(T.fct_items, grid_ctas));
   switch (tb) {
