@@ -325,17 +325,13 @@ constexpr int kFctSegment = 1;
 
 void choose_launch_shape(ymkh_ctx* c) {
   cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->device);
-  // Strip width.  Where rows come by TMA (periodic x, NX even) the 128-wide
-  // form is the faster one from NX = 128 up (FCT us, NZ x NX, 128- against
-  // 64-wide strips: 64 x 128 23 / 29, 256 x 512 47 / 48, 256 x 768 56 / 73,
-  // 2048 x 128 85 / 96) and below that from NZ = 256 up (512 x 64 35 / 44,
-  // but 64 x 96 28 / 24, where its row start-up shows).  Its element-wise
-  // copies (walls, odd NX) are issued by four of its sixteen warps: there it
-  // takes wide grids to win (walls, 256 x 513 77 / 63, 64 x 769 47 / 51,
-  // 512 x 1025 140 / 157).
-  const bool tma = c->sp.periodic_x && c->nx % 2 == 0;
-  const bool wide = tma ? (c->nx >= 128 || c->nz >= 256) : c->nx >= 768;
-  c->fct_tx = wide ? 128 : (c->nx >= 128 ? 64 : 32);
+  // Strip width: 128 from NX = 128 or NZ = 128 up, below 32, where the 128-wide
+  // form's start-up shows (FCT us, NZ x NX, 128- against the better of 64- and
+  // 32-wide strips: 64 x 128 23 / 28, 256 x 512 37 / 52, 128 x 96 27 / 28, 512 x
+  // 64 35 / 38, but 64 x 96 27 / 25, 32 x 48 29 / 23; element copies, walls 64 x
+  // 200 28 / 31, 243 x 371 47 / 58, 1000 x 300 87 / 118, 64 x 96 29 / 29, odd
+  // periodic 243 x 371 47 / 53, 33 x 47 29 / 24).
+  c->fct_tx = c->nx >= 128 || c->nz >= 128 ? 128 : 32;
   const int fct_per_sm = std::max(1, fct_ctas_per_sm(c->fct_tx));
   c->fct_grid = c->sms * fct_per_sm;
   // segments are the FCT's unit of load balance: each CTA runs a contiguous

@@ -146,6 +146,15 @@ __device__ __forceinline__ int xmap(int x, int nx, int periodic) {
   }
   return x < 0 ? 0 : (x >= nx ? nx - 1 : x);
 }
+// Column staged at shear index x.  At a wall the ghost columns that outputs read,
+// four at most, are copies of the edge cell (xmap); the positions past them are
+// computed with but never reach an output, and take mirrored columns: lanes that
+// copy one and the same element cost far more than lanes copying a row (walls,
+// 128-wide FCT 243 x 371 64 -> 47 us, whose last strip is 11 columns wide).
+__device__ __forceinline__ int stage_x(int x, int nx, int periodic) {
+  if (!periodic && x >= nx + 4) return max(0, 2 * nx + 3 - x);
+  return xmap(x, nx, periodic);
+}
 __device__ __forceinline__ int zclamp(int z, int nz) { return z < 0 ? 0 : (z >= nz ? nz - 1 : z); }
 
 __device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {

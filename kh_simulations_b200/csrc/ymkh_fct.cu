@@ -13,7 +13,8 @@
 //
 // Two forms: fct_strip_kernel (128-wide strips, one warp per variable, further
 // down with its own comment) for all but the smallest grids and for batches,
-// and fct_fused_kernel<32 | 64>, described here.
+// and fct_fused_kernel<32 | 64>, described here (32 for the smallest grids, 64
+// where the caller or the tuner asks for it).
 //
 // Layout: work items are (x-strip, z-segment) pairs; each persistent CTA takes
 // a contiguous block of them and runs each strip's part as one piece.  A strip
@@ -176,7 +177,7 @@ __global__ void __launch_bounds__(4 * TB, 2)
     const int x0 = strip * TO;
 
     if (!bulk)
-      for (int i = tid; i < W; i += NT) xtab[i] = xmap(x0 - 4 + i, nx, p.periodic_x);
+      for (int i = tid; i < W; i += NT) xtab[i] = stage_x(x0 - 4 + i, nx, p.periodic_x);
     // the pz source before the first row is zero, as the pipeline's start
     for (int i = tid; i < 2 * 2 * W; i += NT) wk[(size_t)(i / (2 * W)) * WB_SIZE * W + WB_SZ * W + i % (2 * W)] = 0.0;
     __syncthreads();
@@ -835,7 +836,7 @@ __global__ void __launch_bounds__(F2_NT, 1) fct_strip_kernel(const __grid_consta
       if (box && htid == 0) tensormap_acquire<kFctMaps>(maps);
       const bool patch_l = x0 == 0, patch = box && c.edge;
       const int patch_q = patch_l ? 0 : nx - (x0 - 4);  // position of the first wrapped column
-      if (!bulk) xtab[q] = xmap(x0 - 4 + q, nx, p.periodic_x);
+      if (!bulk) xtab[q] = stage_x(x0 - 4 + q, nx, p.periodic_x);
       // row copies of the piece: source array, its row (z, z-1, z+1), its place in the fluid or field ring
       if (htid < narr) {
         const int a = htid;

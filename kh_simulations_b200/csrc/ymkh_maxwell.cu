@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(MX_NT, YMKH_MX_MINB)
       tensormap_acquire(rd.mx_field);
     }
 
-    for (int i = tid; i < W; i += NT) xtab[i] = xmap(x0 - 2 + i, nx, p.periodic_x);
+    for (int i = tid; i < W; i += NT) xtab[i] = stage_x(x0 - 2 + i, nx, p.periodic_x);
     __syncthreads();
 
     auto issue_row = [&](int q) {
