@@ -51,7 +51,7 @@ PHYSICS = ("k_mode = 1\nalpha_YM = 1.0\nperturb_amp = 0.15\nrun_mode = 6\nV0 = 0
            "lx_override = 20\ncourant_override = 0.4\n")
 BYTES_STEP = 376  # compulsory: read 24 FP64 arrays, write 23 (Az1 frozen)
 L2_BYTES = 126 << 20  # B200 L2
-BYTES_FCT = 288   # fct_fused_kernel: read 12 fluid + 12 field arrays, write 12 fluid
+BYTES_FCT = 288   # fused FCT: read 12 fluid + 12 field arrays, write 12 fluid
 BYTES_MAXWELL = 280  # maxwell_fused_kernel: read 24, write 11 (Az1 frozen)
 
 

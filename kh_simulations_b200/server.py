@@ -127,10 +127,9 @@ class KHServer:
     keep_state: copy each finished run's final state to the host.
     large_cells: runs of at least this many cells fill the GPU on their own
         (one persistent FCT/Maxwell kernel over their tiles already occupies
-        every SM, and the lone-run schedule of 128-wide strips in contiguous
-        blocks is faster than a batch's): they are stepped one at a time in
-        arrival order, in turns with the smaller runs, which advance
-        together as one batch.  0 batches every run.
+        every SM): they are stepped one at a time in arrival order, in turns
+        with the smaller runs, which advance together as one batch.  0
+        batches every run.
     """
 
     def __init__(self, budget_bytes: int, device="cuda", chunk: int = 100, graph_steps: int = 4,
