@@ -314,6 +314,10 @@ __device__ __forceinline__ void mbar_wait(uint64_t* bar, unsigned phase, unsigne
   }
   if (err) atomicOr(err, ERR_WAIT);
 }
+// Orders this thread's ordinary shared-memory writes (stores, completed cp.async)
+// before TMA writes to the same addresses that are requested after a barrier:
+// the two go through different proxies, which a barrier alone does not order.
+__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
   unsigned d = (unsigned)__cvta_generic_to_shared(dst);
   unsigned b = (unsigned)__cvta_generic_to_shared(bar);

@@ -479,7 +479,10 @@ __global__ void __launch_bounds__(4 * TB, 2)
     };
     if (half == 0) rows(HalfC<0>{});
     else rows(HalfC<1>{});
-    if (!bulk) cp_async_wait<0>();
+    if (!bulk) {  // the next piece may take the stages by TMA
+      cp_async_wait<0>();
+      fence_proxy_async();
+    }
   }
 }
 
@@ -950,6 +953,7 @@ __global__ void __launch_bounds__(F2_NT, 1) fct_strip_kernel(const __grid_consta
           const int a = e >> 2, x = patch_q + (e & 3);
           if (x < W) (a < 12 ? fl + a * W : fd + (a - 12) * W)[x] = src[e];
         }
+        fence_proxy_async();  // the slots go back to TMA
       };
       for (int i = 0; i < nrow; ++i) {
         // row i staged
@@ -1048,7 +1052,10 @@ __global__ void __launch_bounds__(F2_NT, 1) fct_strip_kernel(const __grid_consta
         if (lane == 0) mbar_arrive(&co_full[gc & 1u]);
         ++gc;
       }
-      if (!bulk) cp_async_wait<0>();
+      if (!bulk) {  // the next piece may take the slots by TMA
+        cp_async_wait<0>();
+        fence_proxy_async();
+      }
       seq += (unsigned)nrow;
     }
   }

@@ -310,7 +310,10 @@ __global__ void __launch_bounds__(MX_NT, YMKH_MX_MINB)
         }
       }
     }
-    if (!bulk) cp_async_wait<0>();
+    if (!bulk) {  // the next item may take the stages by TMA
+      cp_async_wait<0>();
+      fence_proxy_async();
+    }
   }
 }
 
