@@ -33,7 +33,9 @@ namespace ymkh {
 namespace {
 
 // Lets the stream's next kernel start its launch; the final kernels wait for
-// the partial sums with dependency_wait.
+// the partial sums with dependency_wait.  They take those as plain pointers:
+// const __restrict__ would promise memory that nobody writes while the kernel
+// runs, whose loads may be moved in front of the wait.
 __device__ __forceinline__ void dependency_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -131,7 +133,7 @@ __global__ void __launch_bounds__(DG_THREADS)
 // *out = the total; with err, out[1] = the device error word.
 constexpr int EF_THREADS = 1024;
 __global__ void __launch_bounds__(EF_THREADS)
-    energy_final_kernel(const double* __restrict__ part, int nparts, double* out, const unsigned* err) {
+    energy_final_kernel(double* part, int nparts, double* out, const unsigned* err) {
   dependency_wait();
   double s = 0.0, c = 0.0;
   for (int i = threadIdx.x; i < nparts; i += EF_THREADS) neumaier_merge(s, c, part[2 * i], part[2 * i + 1]);
@@ -211,7 +213,7 @@ __global__ void __launch_bounds__(256)
 // With one: (sum_x w[x] |F| / nz, sum_x w[x] |Fc| / nz), the shear-layer
 // weighted average of resolution_convergence.py:83-86.
 __global__ void __launch_bounds__(1024)
-    mode_amp_final_kernel(const double4* __restrict__ part, int splits, const double* __restrict__ w, int nx, int nz,
+    mode_amp_final_kernel(double4* part, int splits, const double* __restrict__ w, int nx, int nz,
                           double* out) {
   dependency_wait();
   double s0 = 0, s1 = 0;
@@ -335,7 +337,7 @@ __global__ void __launch_bounds__(GA_THREADS, 2)
 
 // One CTA per value: the CTA partials, then the root-mean-square over the N cells.
 __global__ void __launch_bounds__(DG_THREADS)
-    gauss_final_kernel(const double2* __restrict__ part, int nparts, double n_cells, double* out) {
+    gauss_final_kernel(double2* part, int nparts, double n_cells, double* out) {
   dependency_wait();
   double s = 0.0, c = 0.0;
   for (int b = threadIdx.x; b < nparts; b += DG_THREADS) {

@@ -4,6 +4,9 @@ when they are missing, checked in the source (no GPU needed).
 * Shared memory that ordinary stores or cp.async have written is handed to TMA
   only behind ``fence.proxy.async``: a barrier orders the threads, not the two
   proxies.
+* A kernel that starts before its predecessor ends reads what that one writes
+  through plain pointers: ``const __restrict__`` data may be read before the
+  ``griddepcontrol.wait``.
 """
 import re
 from pathlib import Path
@@ -37,3 +40,13 @@ def test_patched_columns_are_fenced_before_tma_retakes_the_slot():
     body = re.search(r"auto patch_row = \[&\]\(.*?\) \{(.*?)\} ;|auto patch_row = \[&\]\(.*?\) \{(.*?)\};", code)
     assert re.search(r"= src\[e\]; \} fence_proxy_async\(\); $", body.group(1) or body.group(2))
     assert re.search(r"if \(patch\) \{ patch_row\([^;]*\); coef_bar\(\); \}", code)
+
+
+def test_dependent_kernels_read_partial_sums_through_plain_pointers():
+    code = _code("ymkh_diag.cu")
+    kernels = re.findall(r"__global__ void __launch_bounds__\(\w+\) (\w+)\(([^)]*)\) \{ dependency_wait\(\);", code)
+    assert sorted(k for k, _ in kernels) == ["energy_final_kernel", "gauss_final_kernel", "mode_amp_final_kernel"]
+    assert {k for k, _ in kernels} == set(re.findall(r"launch_dependent\((\w+_kernel)", code))
+    for _, params in kernels:
+        part = params.split(",")[0]
+        assert part.endswith(" part") and "const" not in part and "__restrict__" not in part, part
