@@ -1156,7 +1156,10 @@ struct ymkh_batch {
   int* dfirst = nullptr;     // items of the fused FCT's CTAs
   std::vector<ColGroup> col;
   std::vector<char> col_member;    // whether the member is in one of the groups
-  std::vector<unsigned> versions;  // of the members' descriptors when the tables were built
+  // of each member when the tables were built: its descriptors' version and the
+  // buffer it stepped from
+  std::vector<unsigned> versions;
+  std::vector<int> cur0;
   int fct_items = 0, mx_items = 0, fx_items = 0, fz_items = 0;
   int tb = 128, fct_grid = 0, mx_grid = 0, fx_grid = 0, fz_grid = 0;
   int fct_mode = YMKH_FCT_FUSED;
@@ -1243,10 +1246,12 @@ int batch_build(ymkh_batch* b, cudaStream_t s) {
   // fused column stages: members sorted by NZ, one table range and launch per NZ
   b->col.clear();
   b->versions.clear();
+  b->cur0.clear();
   std::vector<int> order;
   int n_ok = 0;
   for (int i = 0; i < n; ++i) {
     b->versions.push_back(b->runs[i]->version);
+    b->cur0.push_back(b->runs[i]->cur);
     n_ok += b->runs[i]->col_ok;
   }
   // one launch per NZ for all members that can, once they are several: what a
@@ -1397,7 +1402,10 @@ int ymkh_batch_step(ymkh_batch* b, int nsteps, void* stream) {
   if (nsteps < 0) return set_err(YMKH_EINVAL, "negative step count");
   NvtxRange range("ymkh_batch_step");
   cudaStream_t s = (cudaStream_t)stream;
-  for (size_t i = 0; i < b->versions.size() && !b->dirty; ++i) b->dirty = b->versions[i] != b->runs[i]->version;
+  // the tables no longer hold for a member with new parameters or arrays, or one
+  // whose state was put into the other buffer (set anew, or stepped alone)
+  for (size_t i = 0; i < b->versions.size() && !b->dirty; ++i)
+    b->dirty = b->versions[i] != b->runs[i]->version || b->runs[i]->cur != (b->cur0[i] ^ b->parity);
   if (b->dirty) { int rc = batch_build(b, s); if (rc) return rc; }
   int done = 0;
   const bool graphs = s != nullptr && b->graph_steps >= 2 && !b->runs.empty();
