@@ -130,7 +130,9 @@ int ymkh_last_error(char* buf, size_t n);
  * builds the FP32-phase twiddle table on the device. */
 int ymkh_create(const ymkh_grid* grid, const ymkh_params* params, ymkh_ctx** out);
 
-/* Updates the step parameters of an existing context (same grid). */
+/* Updates the step parameters of an existing context (same grid).  Parameters
+ * refused with YMKH_EINVAL leave the run as it was; after any other error it
+ * has the new parameters but no band filters (their memory could not be had). */
 int ymkh_set_params(ymkh_ctx* ctx, const ymkh_params* params);
 
 /* Binds caller-owned device arrays (YMFieldPtrs / YMFluidPtrs without the

@@ -253,6 +253,30 @@ int setup_tf32(ymkh_ctx* c) {
   return 0;
 }
 
+// Twiddles and scratch of the bands of c->prm.
+int setup_bands(ymkh_ctx* c, int nb, const int* lo, const int* hi) {
+  size_t maxJ = 0;
+  for (int b = 0; b < nb; ++b) {
+    c->lo[b] = lo[b]; c->hi[b] = hi[b]; c->J[b] = 2 * (hi[b] - lo[b] + 1);
+    CK(cudaMalloc(&c->W[b], (size_t)c->nz * c->J[b] * sizeof(double)), "cudaMalloc twiddles");
+    CK(launch_twiddles(c->W[b], c->nz, lo[b], hi[b], c->J[b], 0), "twiddle kernel");
+    g_launches++;
+    maxJ = std::max(maxJ, (size_t)c->J[b]);
+  }
+  c->nb = nb;
+  if (nb && c->prm.filter_engine == YMKH_FILTER_TF32X3) {
+    int rc = setup_tf32(c);
+    if (rc) return rc;
+  } else if (nb) {
+    CK(cudaMalloc(&c->coef, 21 * maxJ * (size_t)c->nx * sizeof(double)), "cudaMalloc band coefficients");
+  }
+  // the twiddle tables and images are built on the legacy default stream:
+  // wait for that stream only, not for other streams' work in flight (a
+  // server creates runs while others step)
+  CK(cudaStreamSynchronize(0), "twiddle setup");
+  return 0;
+}
+
 int setup_params(ymkh_ctx* c, const ymkh_params* p) {
   if (p->dt_step <= 0 || p->dx <= 0 || p->dz <= 0) return set_err(YMKH_EINVAL, "dx, dz, dt_step must be > 0");
   if (p->filter_engine != YMKH_FILTER_DFT && p->filter_engine != YMKH_FILTER_TF32X3)
@@ -267,28 +291,19 @@ int setup_params(ymkh_ctx* c, const ymkh_params* p) {
     if (lo[b] < 0 || hi[b] < lo[b] || hi[b] > 1 << 20) return set_err(YMKH_EINVAL, "bad band [%d, %d]", lo[b], hi[b]);
   drop_graphs(c);
   free_bands(c);
+  // The tables of the column stages, this run's and those of a batch that it is
+  // in, point at the bands just freed: they are built again before the next
+  // step, also when the new bands cannot be had.
+  c->desc_ok = false;
+  ++c->version;
   c->prm = *p;
   fill_step_params(c);
-  size_t maxJ = 0;
-  for (int b = 0; b < nb; ++b) {
-    c->lo[b] = lo[b]; c->hi[b] = hi[b]; c->J[b] = 2 * (hi[b] - lo[b] + 1);
-    CK(cudaMalloc(&c->W[b], (size_t)c->nz * c->J[b] * sizeof(double)), "cudaMalloc twiddles");
-    CK(launch_twiddles(c->W[b], c->nz, lo[b], hi[b], c->J[b], 0), "twiddle kernel");
-    g_launches++;
-    maxJ = std::max(maxJ, (size_t)c->J[b]);
+  const int rc = setup_bands(c, nb, lo, hi);
+  if (rc) {
+    free_bands(c);       // no half of a band list: the run goes on without bands
+    cudaGetLastError();  // reported here, not by the next launch
   }
-  c->nb = nb;
-  if (nb && p->filter_engine == YMKH_FILTER_TF32X3) {
-    int rc = setup_tf32(c);
-    if (rc) return rc;
-  } else if (nb) {
-    CK(cudaMalloc(&c->coef, 21 * maxJ * (size_t)c->nx * sizeof(double)), "cudaMalloc band coefficients");
-  }
-  // the twiddle tables and images are built on the legacy default stream:
-  // wait for that stream only, not for other streams' work in flight (a
-  // server creates runs while others step)
-  CK(cudaStreamSynchronize(0), "twiddle setup");
-  return 0;
+  return rc;
 }
 
 // Maxwell's segment rows for persistent CTAs taking (strip, segment) items
