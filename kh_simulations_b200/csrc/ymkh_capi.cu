@@ -141,8 +141,8 @@ struct ymkh_ctx {
   Tf32Scratch tfs{};                // TF32 engine: G and C^T tile images
   double* zmeans = nullptr;         // TF32 engine with suppress_kz0: z-means the first band takes off
   double* epart = nullptr;   // energy partials
-  double* hres = nullptr;    // results of the diagnostics: a slot of pinned host memory (on first use)
-  double* mcol = nullptr;    // mode amplitude partial sums (allocated on first use)
+  double* hres = nullptr;    // results of the diagnostics: a slot of pinned host memory
+  double* mcol = nullptr;    // mode amplitude partial sums
   double* mweight = nullptr; // x weights of ymkh_circ_amp (NX doubles, allocated on first use)
   double* gpart = nullptr;   // Gauss residual partials (allocated on first use)
   SnapshotQueue* snaps = nullptr;  // snapshot writers (created on first use)
@@ -806,8 +806,11 @@ int ymkh_create(const ymkh_grid* grid, const ymkh_params* params, ymkh_ctx** out
   choose_launch_shape(c);
   CK_CREATE(prepare_column(c->nz), "column kernel attributes");
 #undef CK_CREATE
+  // everything that energy and amplitude calls need, so that a first one in the
+  // middle of a campaign that fills the memory cannot fail for the want of it
   const int np = energy_nparts(c->N);
-  if (cudaMalloc(&c->epart, (size_t)2 * np * sizeof(double)) != cudaSuccess ||
+  if (!(c->hres = host_slots().take()) || cudaMalloc(&c->epart, (size_t)2 * np * sizeof(double)) != cudaSuccess ||
+      cudaMalloc(&c->mcol, mode_amp_scratch(c->nx, c->nz) * sizeof(double)) != cudaSuccess ||
       cudaMalloc(&c->derr, sizeof(unsigned)) != cudaSuccess || cudaMemset(c->derr, 0, sizeof(unsigned)) != cudaSuccess) {
     ymkh_destroy(c);
     return set_err(YMKH_ENOMEM, "cudaMalloc diagnostics");
@@ -1036,17 +1039,10 @@ int ymkh_energy_async(ymkh_ctx* c, double* dev_out, void* stream) {
   return 0;
 }
 
-// Slot of the diagnostics' results.
-static int host_result(ymkh_ctx* c) {
-  if (!c->hres && !(c->hres = host_slots().take())) return set_err(YMKH_ENOMEM, "cudaHostAlloc diagnostics page");
-  return 0;
-}
-
 int ymkh_energy(ymkh_ctx* c, double* host_out, void* stream) {
   if (!host_out) return set_err(YMKH_EINVAL, "null argument");
   if (!c) return set_err(YMKH_EINVAL, "null argument");
   if (!c->bound) return set_err(YMKH_ESTATE, "state not bound");
-  { int rc = host_result(c); if (rc) return rc; }
   cudaStream_t s = (cudaStream_t)stream;
   CK(launch_energy(c->buf[c->cur], c->N, c->epart, c->hres, c->derr, s), "energy kernels");
   g_launches += 2;
@@ -1066,9 +1062,6 @@ int ymkh_circ_amp(ymkh_ctx* c, int pair, int k, const double* host_weight, doubl
   if (pair < 0 || pair > 3) return set_err(YMKH_EINVAL, "pair %d not in 0..3", pair);
   cudaStream_t s = (cudaStream_t)stream;
   const State& st = c->buf[c->cur];
-  { int rc = host_result(c); if (rc) return rc; }
-  if (!c->mcol && cudaMalloc(&c->mcol, mode_amp_scratch(c->nx, c->nz) * sizeof(double)) != cudaSuccess)
-    return set_err(YMKH_ENOMEM, "cudaMalloc mode amplitude scratch");
   const double* w = nullptr;
   if (host_weight) {
     if (!c->mweight && cudaMalloc(&c->mweight, (size_t)c->nx * sizeof(double)) != cudaSuccess)
@@ -1091,7 +1084,6 @@ int ymkh_gauss(ymkh_ctx* c, double* host_out, void* stream) {
   if (!c->bound) return set_err(YMKH_ESTATE, "state not bound");
   const int np = gauss_nparts(c->N);
   const size_t n = (size_t)np * YMKH_GAUSS_NOUT * 2;
-  { int rc = host_result(c); if (rc) return rc; }
   if (!c->gpart && cudaMalloc(&c->gpart, n * sizeof(double)) != cudaSuccess)
     return set_err(YMKH_ENOMEM, "cudaMalloc Gauss partials");
   cudaStream_t s = (cudaStream_t)stream;
