@@ -23,6 +23,8 @@
 #include <cstring>
 #include <cstdarg>
 #include <atomic>
+#include <exception>
+#include <memory>
 #include <mutex>
 #include <vector>
 #include <algorithm>
@@ -62,6 +64,12 @@ struct NvtxRange {
     if (e_ != cudaSuccess) return set_err(YMKH_ECUDA, "%s: %s", what, cudaGetErrorString(e_)); \
   } while (0)
 
+// Ends an entry point written as a function-try-block: no exception (a host
+// allocation that fails) leaves the C boundary.
+#define YMKH_CATCH                                                                          \
+  catch (const std::exception& e_) { return set_err(YMKH_ENOMEM, "host: %s", e_.what()); } \
+  catch (...) { return set_err(YMKH_ENOMEM, "host exception"); }
+
 constexpr int MAX_BANDS = kMaxBands;
 constexpr int kMaxFctCtas = 512;
 
@@ -74,7 +82,7 @@ constexpr int kMaxFctCtas = 512;
 class HostSlots {
  public:
   static constexpr int kDoubles = 32, kPerSlab = 256;
-  double* take() {
+  double* take() try {
     std::lock_guard<std::mutex> lock(mu_);
     for (Slab& s : slabs_)
       if (s.used < kPerSlab)
@@ -83,8 +91,15 @@ class HostSlots {
     void* p = nullptr;
     if (cudaHostAlloc(&p, sizeof(double) * kDoubles * kPerSlab, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess)
       return nullptr;
+    struct Free {
+      void operator()(void* q) const { cudaFreeHost(q); }
+    };
+    std::unique_ptr<void, Free> hold(p);
     slabs_.push_back(Slab{static_cast<double*>(p), 0, std::vector<char>(kPerSlab, 0)});
+    hold.release();
     return give_out(slabs_.back(), 0);
+  } catch (const std::bad_alloc&) {
+    return nullptr;
   }
   void give_back(double* slot) {
     std::lock_guard<std::mutex> lock(mu_);
@@ -778,7 +793,7 @@ long long ymkh_launch_count(void) { return g_launches.load(); }
 
 int ymkh_build_flags(void) { return YMKH_DEBUG ? YMKH_BUILD_DEBUG : 0; }
 
-int ymkh_create(const ymkh_grid* grid, const ymkh_params* params, ymkh_ctx** out) {
+int ymkh_create(const ymkh_grid* grid, const ymkh_params* params, ymkh_ctx** out) try {
   if (!grid || !params || !out) return set_err(YMKH_EINVAL, "null argument");
   if (grid->nx < 4 || grid->nz < 4) return set_err(YMKH_EINVAL, "grid too small (%d x %d)", grid->nx, grid->nz);
   if ((size_t)grid->nx * grid->nz > ((size_t)1 << 34)) return set_err(YMKH_EINVAL, "grid too large");
@@ -817,14 +832,14 @@ int ymkh_create(const ymkh_grid* grid, const ymkh_params* params, ymkh_ctx** out
   }
   *out = c;
   return 0;
-}
+} YMKH_CATCH
 
-int ymkh_set_params(ymkh_ctx* c, const ymkh_params* p) {
+int ymkh_set_params(ymkh_ctx* c, const ymkh_params* p) try {
   if (!c || !p) return set_err(YMKH_EINVAL, "null argument");
   int rc = setup_params(c, p);
   if (rc) return rc;
   return upload_desc(c);
-}
+} YMKH_CATCH
 
 static State make_state(double* const f[12], double* const a[6], double* const b[6]) {
   State s{};
@@ -847,7 +862,7 @@ static bool state_ok(const State& s) {
 }
 
 int ymkh_bind_state(ymkh_ctx* c, double* const fields[YMKH_NFIELDS], double* const fluidA[YMKH_NFLUID],
-                    double* const fluidB[YMKH_NFLUID]) {
+                    double* const fluidB[YMKH_NFLUID]) try {
   if (!c || !fields || !fluidA || !fluidB) return set_err(YMKH_EINVAL, "null argument");
   State s = make_state(fields, fluidA, fluidB);
   if (!state_ok(s)) return set_err(YMKH_EINVAL, "null state array");
@@ -867,11 +882,11 @@ int ymkh_bind_state(ymkh_ctx* c, double* const fields[YMKH_NFIELDS], double* con
   c->bound = true;
   c->aligned16 = aligned16(c->buf[0]) && aligned16(c->buf[1]);
   return upload_desc(c);
-}
+} YMKH_CATCH
 
 // Zero-copy form: the caller provides both buffers; after ymkh_step the
 // current state is in buffer ymkh_current_buffer().
-int ymkh_bind_state2(ymkh_ctx* c, double* const* state0, double* const* state1) {
+int ymkh_bind_state2(ymkh_ctx* c, double* const* state0, double* const* state1) try {
   if (!c || !state0 || !state1) return set_err(YMKH_EINVAL, "null argument");
   State s0 = make_state(state0, state0 + 12, state0 + 18);
   State s1 = make_state(state1, state1 + 12, state1 + 18);
@@ -885,11 +900,11 @@ int ymkh_bind_state2(ymkh_ctx* c, double* const* state0, double* const* state1) 
   c->bound = true;
   c->aligned16 = aligned16(s0) && aligned16(s1);
   return upload_desc(c);
-}
+} YMKH_CATCH
 
 // Reads (and clears) the device error word set by in-kernel waits that ran
 // out of polls; synchronises the stream.
-int ymkh_check(ymkh_ctx* c, void* stream) {
+int ymkh_check(ymkh_ctx* c, void* stream) try {
   if (!c) return set_err(YMKH_EINVAL, "null context");
   unsigned h = 0;
   CK(cudaMemcpyAsync(&h, c->derr, sizeof h, cudaMemcpyDeviceToHost, (cudaStream_t)stream), "error word D2H");
@@ -901,18 +916,18 @@ int ymkh_check(ymkh_ctx* c, void* stream) {
                    h);
   }
   return 0;
-}
+} YMKH_CATCH
 
 int ymkh_current_buffer(ymkh_ctx* c) { return c ? c->cur : -1; }
 
-int ymkh_set_current_buffer(ymkh_ctx* c, int which) {
+int ymkh_set_current_buffer(ymkh_ctx* c, int which) try {
   if (!c || (which != 0 && which != 1)) return set_err(YMKH_EINVAL, "bad buffer index");
   if (!c->dual && which == 1) return set_err(YMKH_ESTATE, "buffer 1 is library-owned");
   c->cur = which;
   return 0;
-}
+} YMKH_CATCH
 
-int ymkh_init(ymkh_ctx* c, const ymkh_init_params* ip, void* stream) {
+int ymkh_init(ymkh_ctx* c, const ymkh_init_params* ip, void* stream) try {
   if (!c || !ip) return set_err(YMKH_EINVAL, "null argument");
   if (!c->bound) return set_err(YMKH_ESTATE, "state not bound");
   cudaStream_t s = (cudaStream_t)stream;
@@ -944,9 +959,9 @@ int ymkh_init(ymkh_ctx* c, const ymkh_init_params* ip, void* stream) {
   }
   CK(e, "init kernel");
   return 0;
-}
+} YMKH_CATCH
 
-int ymkh_step(ymkh_ctx* c, int nsteps, void* stream) {
+int ymkh_step(ymkh_ctx* c, int nsteps, void* stream) try {
   if (!c) return set_err(YMKH_EINVAL, "null context");
   if (!c->bound) return set_err(YMKH_ESTATE, "state not bound");
   if (nsteps < 0) return set_err(YMKH_EINVAL, "negative step count");
@@ -972,41 +987,41 @@ int ymkh_step(ymkh_ctx* c, int nsteps, void* stream) {
   }
   if (!c->dual && c->cur == 1) return copy_back(c, s);
   return 0;
-}
+} YMKH_CATCH
 
-int ymkh_set_graph_steps(ymkh_ctx* c, int n) {
+int ymkh_set_graph_steps(ymkh_ctx* c, int n) try {
   if (!c || n < 0 || (n % 2) != 0) return set_err(YMKH_EINVAL, "graph step count must be even and >= 0");
   drop_graphs(c);
   c->graph_steps = n;
   return 0;
-}
+} YMKH_CATCH
 
-int ymkh_set_fct_shape(ymkh_ctx* c, int tx, int seg) {
+int ymkh_set_fct_shape(ymkh_ctx* c, int tx, int seg) try {
   if (!c || (tx != 32 && tx != 64 && tx != 128) || seg < 1) return set_err(YMKH_EINVAL, "bad FCT launch shape");
   drop_graphs(c);
   c->fct_tx = tx;
   c->fct_seg = seg;
   c->fct_grid = c->sms * std::max(1, fct_ctas_per_sm(tx));
   return upload_desc(c);
-}
+} YMKH_CATCH
 
-int ymkh_set_fct_mode(ymkh_ctx* c, int mode) {
+int ymkh_set_fct_mode(ymkh_ctx* c, int mode) try {
   if (!c || (mode != YMKH_FCT_FUSED && mode != YMKH_FCT_SPLIT)) return set_err(YMKH_EINVAL, "bad FCT mode");
   drop_graphs(c);
   c->fct_mode = mode;
   return upload_desc(c);
-}
+} YMKH_CATCH
 
-int ymkh_get_fct_shape(ymkh_ctx* c, int* tx, int* seg) {
+int ymkh_get_fct_shape(ymkh_ctx* c, int* tx, int* seg) try {
   if (!c) return set_err(YMKH_EINVAL, "null context");
   if (tx) *tx = c->fct_tx;
   if (seg) *seg = c->fct_seg;
   return 0;
-}
+} YMKH_CATCH
 
 // Runs nsteps plain (uncaptured) steps with an event between stages and
 // accumulates the device time of each stage into out_ms[0..ST_COUNT).
-int ymkh_stage_times(ymkh_ctx* c, int nsteps, void* stream, float* out_ms, int nout) {
+int ymkh_stage_times(ymkh_ctx* c, int nsteps, void* stream, float* out_ms, int nout) try {
   if (!c || !out_ms || nout < ST_COUNT) return set_err(YMKH_EINVAL, "bad arguments");
   if (!c->bound) return set_err(YMKH_ESTATE, "state not bound");
   cudaStream_t s = (cudaStream_t)stream;
@@ -1029,17 +1044,17 @@ int ymkh_stage_times(ymkh_ctx* c, int nsteps, void* stream, float* out_ms, int n
   for (int i = 0; i <= ST_COUNT; ++i) cudaEventDestroy(c->ev[i]);
   if (!rc && !c->dual && c->cur == 1) rc = copy_back(c, s);
   return rc;
-}
+} YMKH_CATCH
 
-int ymkh_energy_async(ymkh_ctx* c, double* dev_out, void* stream) {
+int ymkh_energy_async(ymkh_ctx* c, double* dev_out, void* stream) try {
   if (!c || !dev_out) return set_err(YMKH_EINVAL, "null argument");
   if (!c->bound) return set_err(YMKH_ESTATE, "state not bound");
   CK(launch_energy(c->buf[c->cur], c->N, c->epart, dev_out, nullptr, (cudaStream_t)stream), "energy kernels");
   g_launches += 2;
   return 0;
-}
+} YMKH_CATCH
 
-int ymkh_energy(ymkh_ctx* c, double* host_out, void* stream) {
+int ymkh_energy(ymkh_ctx* c, double* host_out, void* stream) try {
   if (!host_out) return set_err(YMKH_EINVAL, "null argument");
   if (!c) return set_err(YMKH_EINVAL, "null argument");
   if (!c->bound) return set_err(YMKH_ESTATE, "state not bound");
@@ -1049,13 +1064,13 @@ int ymkh_energy(ymkh_ctx* c, double* host_out, void* stream) {
   CK(cudaStreamSynchronize(s), "energy sync");
   *host_out = c->hres[0];
   return c->hres[1] != 0.0 ? ymkh_check(c, stream) : 0;  // reports and clears the error word
-}
+} YMKH_CATCH
 
-int ymkh_mode_amp(ymkh_ctx* c, int k, double* host_out2, void* stream) {
+int ymkh_mode_amp(ymkh_ctx* c, int k, double* host_out2, void* stream) try {
   return ymkh_circ_amp(c, YMKH_PAIR_AZ, k, nullptr, host_out2, stream);
-}
+} YMKH_CATCH
 
-int ymkh_circ_amp(ymkh_ctx* c, int pair, int k, const double* host_weight, double* host_out2, void* stream) {
+int ymkh_circ_amp(ymkh_ctx* c, int pair, int k, const double* host_weight, double* host_out2, void* stream) try {
   if (!c || !host_out2) return set_err(YMKH_EINVAL, "null argument");
   if (!c->bound) return set_err(YMKH_ESTATE, "state not bound");
   static const int re_of[4] = {AZ2, BY2, EX2, EZ2};
@@ -1077,9 +1092,9 @@ int ymkh_circ_amp(ymkh_ctx* c, int pair, int k, const double* host_weight, doubl
   host_out2[0] = c->hres[0];
   host_out2[1] = c->hres[1];
   return 0;
-}
+} YMKH_CATCH
 
-int ymkh_gauss(ymkh_ctx* c, double* host_out, void* stream) {
+int ymkh_gauss(ymkh_ctx* c, double* host_out, void* stream) try {
   if (!c || !host_out) return set_err(YMKH_EINVAL, "null argument");
   if (!c->bound) return set_err(YMKH_ESTATE, "state not bound");
   const int np = gauss_nparts(c->N);
@@ -1093,9 +1108,9 @@ int ymkh_gauss(ymkh_ctx* c, double* host_out, void* stream) {
   CK(cudaStreamSynchronize(s), "Gauss sync");
   for (int i = 0; i < YMKH_GAUSS_NOUT; ++i) host_out[i] = c->hres[i];
   return 0;
-}
+} YMKH_CATCH
 
-int ymkh_snapshot(ymkh_ctx* c, const char* path, int format, void* stream) {
+int ymkh_snapshot(ymkh_ctx* c, const char* path, int format, void* stream) try {
   if (!c || !path) return set_err(YMKH_EINVAL, "null argument");
   if (!c->bound) return set_err(YMKH_ESTATE, "state not bound");
   if (format != YMKH_SNAP_CSV && format != YMKH_SNAP_FP64) return set_err(YMKH_EINVAL, "snapshot format %d", format);
@@ -1104,17 +1119,17 @@ int ymkh_snapshot(ymkh_ctx* c, const char* path, int format, void* stream) {
   const int rc = snapshot_submit(c->snaps, c->buf[c->cur], c->nx, c->nz, c->prm.dx, c->prm.dz, path, format,
                                  (cudaStream_t)stream, err);
   return rc ? set_err(rc, "%s", err.c_str()) : 0;
-}
+} YMKH_CATCH
 
-int ymkh_snapshot_wait(ymkh_ctx* c) {
+int ymkh_snapshot_wait(ymkh_ctx* c) try {
   if (!c) return set_err(YMKH_EINVAL, "null context");
   if (!c->snaps) return 0;
   std::string err;
   const int rc = snapshot_wait(c->snaps, err);
   return rc ? set_err(rc, "%s", err.c_str()) : 0;
-}
+} YMKH_CATCH
 
-int ymkh_destroy(ymkh_ctx* c) {
+int ymkh_destroy(ymkh_ctx* c) try {
   if (!c) return 0;
   if (c->snaps) snapshot_queue_destroy(c->snaps);  // waits for its writers
   drop_graphs(c);
@@ -1130,9 +1145,9 @@ int ymkh_destroy(ymkh_ctx* c) {
   if (c->xscratch) cudaFree(c->xscratch);
   delete c;
   return 0;
-}
+} YMKH_CATCH
 
-int ymkh_twiddles(int nz, int m_lo, int m_hi, float* cos_out, float* sin_out) {
+int ymkh_twiddles(int nz, int m_lo, int m_hi, float* cos_out, float* sin_out) try {
   if (nz < 1 || m_lo < 0 || m_hi < m_lo || !cos_out || !sin_out) return set_err(YMKH_EINVAL, "bad arguments");
   const size_t n = (size_t)(m_hi - m_lo + 1) * nz;
   float *dc = nullptr, *ds = nullptr;
@@ -1146,7 +1161,7 @@ int ymkh_twiddles(int nz, int m_lo, int m_hi, float* cos_out, float* sin_out) {
   cudaFree(ds);
   CK(e, "twiddle table");
   return 0;
-}
+} YMKH_CATCH
 
 // ------------------------------------------------------------------ batches
 // Runs of any sizes advance together: one FCT and one Maxwell launch per step
@@ -1346,7 +1361,7 @@ int batch_step_once(ymkh_batch* b, cudaStream_t s) {
 
 }  // namespace
 
-int ymkh_batch_create(ymkh_batch** out) {
+int ymkh_batch_create(ymkh_batch** out) try {
   if (!out) return set_err(YMKH_EINVAL, "null argument");
   ymkh_batch* b = new ymkh_batch();
   int dev = 0, sms = 148;
@@ -1375,36 +1390,36 @@ int ymkh_batch_create(ymkh_batch** out) {
   }
   *out = b;
   return 0;
-}
+} YMKH_CATCH
 
-int ymkh_batch_add(ymkh_batch* b, ymkh_ctx* c) {
+int ymkh_batch_add(ymkh_batch* b, ymkh_ctx* c) try {
   if (!b || !c) return set_err(YMKH_EINVAL, "null argument");
   if (!c->bound) return set_err(YMKH_ESTATE, "run state not bound");
   for (ymkh_ctx* r : b->runs) if (r == c) return set_err(YMKH_EINVAL, "run already in the batch");
   b->runs.push_back(c);
   b->dirty = true;
   return 0;
-}
+} YMKH_CATCH
 
-int ymkh_batch_remove(ymkh_batch* b, ymkh_ctx* c) {
+int ymkh_batch_remove(ymkh_batch* b, ymkh_ctx* c) try {
   if (!b || !c) return set_err(YMKH_EINVAL, "null argument");
   auto it = std::find(b->runs.begin(), b->runs.end(), c);
   if (it == b->runs.end()) return set_err(YMKH_EINVAL, "run not in the batch");
   b->runs.erase(it);
   b->dirty = true;
   return 0;
-}
+} YMKH_CATCH
 
 int ymkh_batch_size(ymkh_batch* b) { return b ? (int)b->runs.size() : -1; }
 
-int ymkh_batch_set_graph_steps(ymkh_batch* b, int n) {
+int ymkh_batch_set_graph_steps(ymkh_batch* b, int n) try {
   if (!b || n < 0 || (n % 2) != 0) return set_err(YMKH_EINVAL, "graph step count must be even and >= 0");
   batch_drop_graph(b);
   b->graph_steps = n;
   return 0;
-}
+} YMKH_CATCH
 
-int ymkh_batch_step(ymkh_batch* b, int nsteps, void* stream) {
+int ymkh_batch_step(ymkh_batch* b, int nsteps, void* stream) try {
   if (!b) return set_err(YMKH_EINVAL, "null batch");
   if (nsteps < 0) return set_err(YMKH_EINVAL, "negative step count");
   NvtxRange range("ymkh_batch_step");
@@ -1466,9 +1481,9 @@ int ymkh_batch_step(ymkh_batch* b, int nsteps, void* stream) {
   // every member's current buffer before the next step.
   if (moved) b->dirty = true;
   return 0;
-}
+} YMKH_CATCH
 
-int ymkh_batch_check(ymkh_batch* b, void* stream) {
+int ymkh_batch_check(ymkh_batch* b, void* stream) try {
   if (!b) return set_err(YMKH_EINVAL, "null batch");
   unsigned h = 0;
   CK(cudaMemcpyAsync(&h, b->derr, sizeof h, cudaMemcpyDeviceToHost, (cudaStream_t)stream), "error word D2H");
@@ -1480,16 +1495,16 @@ int ymkh_batch_check(ymkh_batch* b, void* stream) {
                    h);
   }
   return 0;
-}
+} YMKH_CATCH
 
-int ymkh_batch_set_fct_mode(ymkh_batch* b, int mode) {
+int ymkh_batch_set_fct_mode(ymkh_batch* b, int mode) try {
   if (!b || (mode != YMKH_FCT_FUSED && mode != YMKH_FCT_SPLIT)) return set_err(YMKH_EINVAL, "bad FCT mode");
   b->fct_mode = mode;
   b->dirty = true;
   return 0;
-}
+} YMKH_CATCH
 
-int ymkh_batch_destroy(ymkh_batch* b) {
+int ymkh_batch_destroy(ymkh_batch* b) try {
   if (!b) return 0;
   batch_drop_graph(b);
   if (b->ddesc) cudaFree(b->ddesc);
@@ -1503,7 +1518,7 @@ int ymkh_batch_destroy(ymkh_batch* b) {
   if (b->fork_ev) cudaEventDestroy(b->fork_ev);
   delete b;
   return 0;
-}
+} YMKH_CATCH
 
 }  // extern "C"
 
