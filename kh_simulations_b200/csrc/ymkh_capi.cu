@@ -355,13 +355,17 @@ constexpr int kFctSegment = 1;
 
 void choose_launch_shape(ymkh_ctx* c) {
   cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->device);
-  // Strip width: 128 from NX = 128 or NZ = 128 up, below 32, where the 128-wide
-  // form's start-up shows (FCT us, NZ x NX, 128- against the better of 64- and
-  // 32-wide strips: 64 x 128 23 / 28, 256 x 512 37 / 52, 128 x 96 27 / 28, 512 x
-  // 64 35 / 38, but 64 x 96 27 / 25, 32 x 48 29 / 23; element copies, walls 64 x
-  // 200 28 / 31, 243 x 371 47 / 58, 1000 x 300 87 / 118, 64 x 96 29 / 29, odd
-  // periodic 243 x 371 47 / 53, 33 x 47 29 / 24).
-  c->fct_tx = c->nx >= 128 || c->nz >= 128 ? 128 : 32;
+  // Strip width: 128 from NX = 128 up, and from NX = 64 up with 128 rows or more;
+  // below 32, where the 128-wide form's start-up shows and on narrow grids its
+  // empty lanes and the many short copies of a wrapped row (FCT us, NZ x NX, 128-
+  // against the better of 64- and 32-wide strips: 64 x 128 23 / 28, 256 x 512 37
+  // / 52, 128 x 96 25 / 26, 512 x 96 33 / 38, 2048 x 64 73 / 80, but 64 x 96 27 /
+  // 25, 32 x 48 29 / 23, 512 x 48 36 / 36, 2048 x 48 78 / 63, 2048 x 16 107 / 46,
+  // 128 x 4 90 / 27; from 53 to 63 columns within a tenth of each other; element
+  // copies, walls 64 x 200 28 / 31, 243 x 371 47 / 58, 1000 x 300 87 / 118, 64 x
+  // 96 29 / 29, 2048 x 64 81 / 91, 2048 x 48 85 / 70, odd periodic 243 x 371 47 /
+  // 53, 33 x 47 29 / 24).
+  c->fct_tx = c->nx >= 128 || (c->nx >= 64 && c->nz >= 128) ? 128 : 32;
   const int fct_per_sm = std::max(1, fct_ctas_per_sm(c->fct_tx));
   c->fct_grid = c->sms * fct_per_sm;
   // segments are the FCT's unit of load balance: each CTA runs a contiguous
