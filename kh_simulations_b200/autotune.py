@@ -42,7 +42,8 @@ def lookup(nx: int, nz: int, filtered: bool):
 
 
 def candidates(nx: int, nz: int):
-    tbs = [tb for tb in (32, 64, 128) if nx >= tb - 6]
+    # 32 or 128 is what a run takes by itself, on grids of any width
+    tbs = [tb for tb in (32, 64, 128) if nx >= tb - 6 or tb != 64]
     segs = sorted({s for s in (1, 16, 32, 64, 128) if s <= max(16, nz)})
     return [(tb, s) for tb in tbs for s in segs]
 
