@@ -1188,6 +1188,7 @@ struct ymkh_batch {
   std::vector<int> cur0;
   int fct_items = 0, mx_items = 0, fx_items = 0, fz_items = 0;
   int tb = 128, fct_grid = 0, mx_grid = 0, fx_grid = 0, fz_grid = 0;
+  int fct_grids[3] = {0, 0, 0};    // CTAs of each strip width (kBatchWidth)
   int fct_mode = YMKH_FCT_FUSED;
   unsigned* derr = nullptr;
   bool dirty = true;
@@ -1211,6 +1212,28 @@ void batch_drop_graph(ymkh_batch* b) {
   if (b->gexec) { cudaGraphExecDestroy(b->gexec); b->gexec = nullptr; b->gstream = nullptr; }
 }
 
+// Strip width of a batch: the one whose strips take least time over all rows of
+// its members.  A strip's row costs about as 4, 6 and 9 in 32-, 64- and 128-wide
+// strips (305, 450 and 690 us for 16 runs of 2048 rows), and in the last form
+// one more for every copy past two that fills the window of a narrow grid.  So
+// 128 but for grids of up to 58 columns (step of 16 runs, 32-, 64- and 128-wide:
+// 2048 x 8 692, 826, 2013 us; 2048 x 48 984, 834, 1133; 2048 x 64 1285, 1292,
+// 1070; 64 x 96 73, -, 56; 64 x 48 54, 57, 60).
+constexpr int kBatchWidth[3] = {32, 64, 128}, kBatchRow[3] = {4, 6, 9};
+int pick_batch_width(const std::vector<ymkh_ctx*>& runs) {
+  int best = 2;
+  long long best_cost = 0;
+  for (int k = 2; k >= 0; --k) {
+    long long cost = 0;
+    for (const ymkh_ctx* c : runs) {
+      const int row = kBatchRow[k] + (k == 2 ? std::max(0, kBatchWidth[k] / c->nx - 2) : 0);
+      cost += (long long)row * fct_nstrips(c->nx, kBatchWidth[k]) * c->nz;
+    }
+    if (k == 2 || cost < best_cost) { best = k; best_cost = cost; }
+  }
+  return best;
+}
+
 int batch_build(ymkh_batch* b, cudaStream_t s) {
   const int n = (int)b->runs.size();
   if (n > b->cap) {
@@ -1224,6 +1247,9 @@ int batch_build(ymkh_batch* b, cudaStream_t s) {
     CK(cudaMalloc(&b->ddesc, 2 * (size_t)cap * sizeof(RunDesc)), "cudaMalloc batch descriptors");
     b->cap = cap;
   }
+  const int width = pick_batch_width(b->runs);
+  b->tb = kBatchWidth[width];
+  b->fct_grid = b->fct_grids[width];
   std::vector<RunDesc> h(2 * (size_t)std::max(n, 1));
   std::vector<StripRun> strips;
   std::vector<MxGrid> mg;
@@ -1374,7 +1400,7 @@ int ymkh_batch_create(ymkh_batch** out) try {
   for (int tb : {32, 64, 128}) prepare_fct(tb);
   prepare_maxwell();
   prepare_fct_split();
-  b->fct_grid = sms * std::max(1, fct_ctas_per_sm(b->tb));
+  for (int k = 0; k < 3; ++k) b->fct_grids[k] = sms * std::max(1, fct_ctas_per_sm(kBatchWidth[k]));
   b->mx_grid = sms * std::max(1, maxwell_ctas_per_sm());
   b->fx_grid = sms * std::max(1, fct_split_ctas_per_sm(0)) * 4;
   b->fz_grid = sms * std::max(1, fct_split_ctas_per_sm(1)) * 4;
