@@ -536,6 +536,28 @@ bool col_fused_alone(const ymkh_ctx* c) {
   return stages >= 2 || (c->nb && c->nz <= 128);
 }
 
+// Whether a member of a batch does, where the launch is shared by all members of
+// its NZ: with 64 rows or less, two stages or more, or bands of up to 24 modes
+// in all; wider bands from 129 rows up only beside other stages and up to 256
+// rows.  Past 24 modes the separate band kernels, which run without a column
+// tile's uneven end, are ahead (step us, one kernel against separate ones, 4
+// and 12 runs: 256 x 512 bands of 16 modes 265 / 294, 724 / 830, 24 modes 323 /
+// 344, 881 / 965, 64 modes 611 / 565, 1686 / 1602; 512 x 512 16 modes 530 / 559,
+// 1489 / 1605, 24 modes 645 / 640, 1805 / 1851, 64 modes 1217 / 1069, 3413 /
+// 3117; z-mean and 86 modes 512 x 512 1316 / 1203, but 43 modes 256 x 512 417 /
+// 430; z-mean alone 64 x 768 69 / 77, 128 x 1024 135 / 129, 512 x 512 280 / 261;
+// z-mean and hyperdiffusion 512 x 512 279 / 297).
+constexpr int kColBatchModes = 24;
+bool col_fused_batch(const ymkh_ctx* c) {
+  if (!c->col_ok) return false;
+  const ymkh_params& p = c->prm;
+  const int stages = (p.xi_sponge > 0.0 || p.xi_cut > 0.0) + (p.suppress_kz0 != 0) + (c->nb > 0) + (p.hyp_diff_coeff > 0.0);
+  int modes = 0;
+  for (int b = 0; b < c->nb; ++b) modes += c->J[b] / 2;
+  if (modes > kColBatchModes && c->nz > 128) return stages >= 2 && c->nz <= 256;
+  return modes > 0 || stages >= 2 || c->nz <= 64;
+}
+
 // How the fused FCT's items (strip-major segments) are cut into one contiguous
 // block per CTA.  The launch lasts as long as its slowest CTA, so the cut is
 // the one whose costliest block is cheapest: in units of a fifth of an inner
@@ -655,11 +677,12 @@ void mark(ymkh_ctx* c, int stage, cudaStream_t s) {
   if (c->timing) cudaEventRecord(c->ev[stage], s);
 }
 
-// Stages after the fused FCT and Maxwell launches, on the run's new buffer.
-int post_stages(ymkh_ctx* c, cudaStream_t s) {
+// Stages after the fused FCT and Maxwell launches, on the run's new buffer: as
+// one kernel (fused) or one by one.
+int post_stages(ymkh_ctx* c, bool fused, cudaStream_t s) {
   const State& out = c->buf[1 - c->cur];
   mark(c, ST_POINTWISE, s);
-  if (c->col_fused) {
+  if (fused) {
     mark(c, ST_ZMEAN, s);
     mark(c, ST_BANDS, s);
     CK(launch_column_fused(c->dev->col + (1 - c->cur), 1, c->col_items, c->nz, c->col_smem, s), "column stages");
@@ -736,7 +759,7 @@ int step_once(ymkh_ctx* c, cudaStream_t s) {
   }
   g_launches += 2;
   NvtxRange r("ymkh column stages");
-  int rc = post_stages(c, s);
+  int rc = post_stages(c, c->col_fused, s);
   if (rc) return rc;
   c->cur = 1 - c->cur;
   return 0;
@@ -1306,11 +1329,10 @@ int batch_build(ymkh_batch* b, cudaStream_t s) {
     b->cur0.push_back(b->runs[i]->cur);
     n_ok += b->runs[i]->col_ok;
   }
-  // one launch per NZ for all members that can, once they are several: what a
-  // member loses to its own kernels is less than its launches
+  // up to three members that can go by what each does alone
   b->col_member.assign(n, 0);
   for (int i = 0; i < n; ++i)
-    if (n_ok >= 4 ? b->runs[i]->col_ok : b->runs[i]->col_fused) {
+    if (n_ok >= 4 ? col_fused_batch(b->runs[i]) : b->runs[i]->col_fused) {
       b->col_member[i] = 1;
       order.push_back(i);
     }
@@ -1373,7 +1395,7 @@ int batch_step_once(ymkh_batch* b, cudaStream_t s) {
   for (int i = 0; i < n; ++i) {
     ymkh_ctx* c = b->runs[i];
     if (separate(i)) {
-      int rc = post_stages(c, na > 1 ? b->aux[job % na] : s);
+      int rc = post_stages(c, false, na > 1 ? b->aux[job % na] : s);
       if (rc) return rc;
       ++job;
     }
