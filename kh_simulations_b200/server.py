@@ -31,8 +31,10 @@ BYTES_PER_CELL_STATE = 2 * 24 * 8  # two 24-array FP64 buffers
 
 def footprint(cfg: RunConfig) -> int:
     """Device bytes a run holds while resident: both state buffers, the
-    band-filter twiddles and coefficient scratch of its filter engine,
-    diagnostics (the allocations of include/ymkh.h's context)."""
+    band-filter twiddles and coefficient scratch of its filter engine, the
+    kernels' tables, and the scratch of all its diagnostics (the allocations of
+    include/ymkh.h's context, those of a first ymkh_gauss or weighted
+    ymkh_circ_amp included)."""
     d = derive(cfg)
     cells = d.nx * d.nz
     fp = BYTES_PER_CELL_STATE * cells
@@ -47,10 +49,18 @@ def footprint(cfg: RunConfig) -> int:
             jpad = [-(-j // 128) * 128 for j in js]
             fp += sum(4 * jp * zpad * 4 for jp in jpad)
             fp += 2 * 21 * xpad * zpad * 4 + 2 * 21 * xpad * max(jpad) * 4
+            if cfg.suppress_kz0:
+                fp += 12 * d.nx * 8  # z-means on their way to the filter
         else:
             fp += 21 * max(js) * d.nx * 8  # FP64 coefficients
-    fp += 64 * 1024 + 16 * d.nx
-    return fp
+    # partial sums (ymkh_diag.cu): 16 bytes per energy CTA, 32 per column and row
+    # range of the amplitudes, 256 per Gauss CTA; the amplitudes' weights
+    energy_ctas = max(-(-cells // (256 * 16)), min(-(-cells // 256), 592))
+    gauss_ctas = max(-(-cells // (128 * 16)), min(-(-cells // 128), 592))
+    tiles = -(-d.nx // 32)
+    ranges = min(max(1, min(-(-592 // tiles), 32)), -(-d.nz // 64))
+    fp += 16 * energy_ctas + 32 * d.nx * ranges + 256 * gauss_ctas + 8 * d.nx
+    return fp + 64 * 1024
 
 
 @dataclass
