@@ -520,7 +520,9 @@ cudaError_t launch_band(const ArrayList& arrs, int narr, const double* W, int ld
   // the fewest modes (us at 256 x 512, modes 86..128: 105 against 112 with
   // halving to four; 512 x 512 320 against 347); beyond, the most that fit,
   // which read the array least (1024 x 2048 3.66 ms against 3.91).
-  const long long slots = 148 * 4;
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const long long slots = sms * 4;
   auto turns = [&](int m) { return ((long long)((M + m - 1) / m) * nxb * narr + slots - 1) / slots; };
   int bm = std::min(BC_BM, M);
   if (turns(bm) <= 4)

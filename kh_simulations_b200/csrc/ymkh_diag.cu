@@ -83,7 +83,8 @@ __device__ __forceinline__ void neumaier_block(double& s, double& c) {
 }
 
 // Cells per thread of the partial sums: `most` on a grid that gives every SM
-// four CTAs that way, fewer below.
+// four CTAs that way, fewer below.  A constant, not the device's SMs: the order of
+// the sums, and with it their last bits, depends on the grid size alone.
 constexpr int DG_THREADS = 256;
 constexpr int DG_CTAS = 148 * 4;
 int cells_per_thread(size_t N, int most) {
