@@ -364,12 +364,14 @@ __device__ __forceinline__ void stage_twiddles(double2* tw, const double* __rest
 }
 
 // C[2m + {0, 1}][x] for modes [m0, m0 + bm) of one array: the running sums of
-// the block's modes stay in shared memory, each thread's own.
-__global__ void __launch_bounds__(BC_NT)
-    band_coef_kernel(const __grid_constant__ ArrayList arrs, const double* __restrict__ W, int ldw, int M, int bm,
-                     double* __restrict__ C, int nx, int nz, double inv2) {
-  constexpr int NC = BC_NC, NT = BC_NT;
-  extern __shared__ __align__(16) double2 band_smem[];
+// the block's modes stay in shared memory, each thread's own.  NC columns a
+// thread: one where 64 columns or fewer are left, so that no thread sums a column
+// that is not there (2048 x 40, modes 683..1024: 722 us against 1182 with two;
+// 1024 x 40 225 against 347).
+template <int NC>
+__device__ __forceinline__ void band_coef(const ArrayList& arrs, const double* __restrict__ W, int ldw, int M, int bm,
+                                          double* __restrict__ C, int nx, int nz, double inv2, double2* band_smem) {
+  constexpr int NT = BC_NT;
   double2* const tw = band_smem;                                              // [2][BD_CH][bm]
   double2* const sum = band_smem + (size_t)2 * BD_CH * bm + threadIdx.x;      // [bm][BD_TX]
   const int m0 = blockIdx.x * bm, x0 = blockIdx.y * BD_TX + threadIdx.x, k = blockIdx.z;
@@ -438,14 +440,21 @@ __global__ void __launch_bounds__(BC_NT)
       }
 }
 
+__global__ void __launch_bounds__(BC_NT)
+    band_coef_kernel(const __grid_constant__ ArrayList arrs, const double* __restrict__ W, int ldw, int M, int bm,
+                     double* __restrict__ C, int nx, int nz, double inv2) {
+  extern __shared__ __align__(16) double2 band_smem[];
+  if (nx - (int)blockIdx.y * BD_TX <= BC_NT) band_coef<1>(arrs, W, ldw, M, bm, C, nx, nz, inv2, band_smem);
+  else band_coef<BC_NC>(arrs, W, ldw, M, bm, C, nx, nz, inv2, band_smem);
+}
+
 // v[z][x] -= sum over the band's modes in order of (A_m cos_m(z) + B_m sin_m(z)),
 // 32 rows and 128 columns per CTA, 16 x 2 of them in a thread's registers: a
 // twiddle pair then serves eight FP64 instructions.
-constexpr int BA_NT = 128, BA_RZ = 16, BA_NC = 2;
-__global__ void __launch_bounds__(BA_NT)
-    band_apply_kernel(const __grid_constant__ ArrayList arrs, const double* __restrict__ W, int ldw, int M,
-                      const double* __restrict__ C, int nx, int nz) {
-  __shared__ __align__(16) double2 tw[2][BD_CH * BA_BM];
+constexpr int BA_NT = 128, BA_RZ = 16;
+template <int BA_NC>  // columns per thread, as in band_coef
+__device__ __forceinline__ void band_apply(const ArrayList& arrs, const double* __restrict__ W, int ldw, int M,
+                                           const double* __restrict__ C, int nx, int nz, double2 (*tw)[BD_CH * BA_BM]) {
   const int zh = (threadIdx.x >> 6) * BA_RZ;
   const int z0 = blockIdx.x * BD_CH, x0 = blockIdx.y * BD_TX + (threadIdx.x & 63), k = blockIdx.z;
   const double* c = C + (size_t)k * 2 * M * nx;
@@ -508,6 +517,14 @@ __global__ void __launch_bounds__(BA_NT)
 #pragma unroll
       for (int i = 0; i < BA_RZ; ++i)
         if (z0 + zh + i < nz) g[(size_t)(z0 + zh + i) * nx + n * 64] -= d[n][i];
+}
+
+__global__ void __launch_bounds__(BA_NT)
+    band_apply_kernel(const __grid_constant__ ArrayList arrs, const double* __restrict__ W, int ldw, int M,
+                      const double* __restrict__ C, int nx, int nz) {
+  __shared__ __align__(16) double2 tw[2][BD_CH * BA_BM];
+  if (nx - (int)blockIdx.y * BD_TX <= 64) band_apply<1>(arrs, W, ldw, M, C, nx, nz, tw);
+  else band_apply<2>(arrs, W, ldw, M, C, nx, nz, tw);
 }
 
 size_t band_coef_smem(int bm) { return sizeof(double2) * (size_t)bm * (2 * BD_CH + BD_TX); }
