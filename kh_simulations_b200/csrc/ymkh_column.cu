@@ -510,13 +510,21 @@ __device__ __forceinline__ void band_apply(const ArrayList& arrs, const double* 
       }
     }
   }
+  // A column's rows are all read before the first is written: the compiler may
+  // not move a read past a write whose row it cannot tell apart, and one after
+  // the other they took longer than a band of few modes (filter at 1024 x 768, one
+  // mode: 108 us against 180, 13 modes 207 against 272).
   double* g = arrs.p[k] + x0;
 #pragma unroll
   for (int n = 0; n < BA_NC; ++n)
-    if (x0 + n * 64 < nx)
+    if (x0 + n * 64 < nx) {
+      double v[BA_RZ];
+#pragma unroll
+      for (int i = 0; i < BA_RZ; ++i) v[i] = z0 + zh + i < nz ? g[(size_t)(z0 + zh + i) * nx + n * 64] : 0.0;
 #pragma unroll
       for (int i = 0; i < BA_RZ; ++i)
-        if (z0 + zh + i < nz) g[(size_t)(z0 + zh + i) * nx + n * 64] -= d[n][i];
+        if (z0 + zh + i < nz) g[(size_t)(z0 + zh + i) * nx + n * 64] = v[i] - d[n][i];
+    }
 }
 
 __global__ void __launch_bounds__(BA_NT)
