@@ -368,13 +368,14 @@ __device__ __forceinline__ void stage_twiddles(double2* tw, const double* __rest
 // thread: one where 64 columns or fewer are left, so that no thread sums a column
 // that is not there (2048 x 40, modes 683..1024: 722 us against 1182 with two;
 // 1024 x 40 225 against 347).
-template <int NC>
+template <int NC, bool AHEAD>
 __device__ __forceinline__ void band_coef(const ArrayList& arrs, const double* __restrict__ W, int ldw, int M, int bm,
-                                          double* __restrict__ C, int nx, int nz, double inv2, double2* band_smem) {
-  constexpr int NT = BC_NT;
+                                          double* __restrict__ C, int xb, int nx, int nz, double inv2,
+                                          double2* band_smem) {
+  constexpr int NT = BC_NT, TX = NC * NT;
   double2* const tw = band_smem;                                              // [2][BD_CH][bm]
-  double2* const sum = band_smem + (size_t)2 * BD_CH * bm + threadIdx.x;      // [bm][BD_TX]
-  const int m0 = blockIdx.x * bm, x0 = blockIdx.y * BD_TX + threadIdx.x, k = blockIdx.z;
+  double2* const sum = band_smem + (size_t)2 * BD_CH * bm + threadIdx.x;      // [bm][TX]
+  const int m0 = blockIdx.x * bm, x0 = xb + threadIdx.x, k = blockIdx.z;
   const double* g = arrs.p[k] + x0;
   bool in[NC];
 #pragma unroll
@@ -382,10 +383,9 @@ __device__ __forceinline__ void band_coef(const ArrayList& arrs, const double* _
   const int nm = min(bm, M - m0), nch = (nz + BD_CH - 1) / BD_CH;
   for (int m = 0; m < nm; ++m)
 #pragma unroll
-    for (int n = 0; n < NC; ++n) sum[m * BD_TX + n * NT] = make_double2(0.0, 0.0);
+    for (int n = 0; n < NC; ++n) sum[m * TX + n * NT] = make_double2(0.0, 0.0);
   stage_twiddles<NT>(tw, W, ldw, 0, m0, bm, nz, M);
-  for (int ch = 0; ch < nch; ++ch) {
-    double f[NC][BD_CH];
+  auto rows = [&](double(&f)[NC][BD_CH], int ch) {
 #pragma unroll
     for (int i = 0; i < BD_CH; ++i)
 #pragma unroll
@@ -393,6 +393,20 @@ __device__ __forceinline__ void band_coef(const ArrayList& arrs, const double* _
         const int z = ch * BD_CH + i;
         f[n][i] = (in[n] && z < nz) ? g[(size_t)z * nx + n * NT] : 0.0;
       }
+  };
+  double next[NC][BD_CH];
+  if (AHEAD) rows(next, 0);
+  for (int ch = 0; ch < nch; ++ch) {
+    double f[NC][BD_CH];
+    if (AHEAD) {
+#pragma unroll
+      for (int i = 0; i < BD_CH; ++i)
+#pragma unroll
+        for (int n = 0; n < NC; ++n) f[n][i] = next[n][i];
+      if (ch + 1 < nch) rows(next, ch + 1);
+    } else {
+      rows(f, ch);
+    }
     cp_async_wait<0>();
     __syncthreads();  // this chunk's twiddles are there, the other buffer is free
     if (ch + 1 < nch) stage_twiddles<NT>(tw + ((ch + 1) & 1) * BD_CH * bm, W, ldw, (ch + 1) * BD_CH, m0, bm, nz, M);
@@ -420,10 +434,10 @@ __device__ __forceinline__ void band_coef(const ArrayList& arrs, const double* _
             sc[n][lvl] = c;
             ss[n][lvl] = s;
           } else {  // warp sums added in warp order from 0.0
-            double2 S = sum[m * BD_TX + n * NT];
+            double2 S = sum[m * TX + n * NT];
             S.x = S.x + c;
             S.y = S.y + s;
-            sum[m * BD_TX + n * NT] = S;
+            sum[m * TX + n * NT] = S;
           }
         }
       }
@@ -434,7 +448,7 @@ __device__ __forceinline__ void band_coef(const ArrayList& arrs, const double* _
   for (int n = 0; n < NC; ++n)
     if (in[n])
       for (int m = 0; m < nm; ++m) {
-        const double2 S = sum[m * BD_TX + n * NT];
+        const double2 S = sum[m * TX + n * NT];
         Ck[(size_t)(2 * m) * nx + n * NT] = S.x * inv2;
         Ck[(size_t)(2 * m + 1) * nx + n * NT] = S.y * inv2;
       }
@@ -444,8 +458,17 @@ __global__ void __launch_bounds__(BC_NT)
     band_coef_kernel(const __grid_constant__ ArrayList arrs, const double* __restrict__ W, int ldw, int M, int bm,
                      double* __restrict__ C, int nx, int nz, double inv2) {
   extern __shared__ __align__(16) double2 band_smem[];
-  if (nx - (int)blockIdx.y * BD_TX <= BC_NT) band_coef<1>(arrs, W, ldw, M, bm, C, nx, nz, inv2, band_smem);
-  else band_coef<BC_NC>(arrs, W, ldw, M, bm, C, nx, nz, inv2, band_smem);
+  const int xb = blockIdx.y * BD_TX;
+  if (nx - xb <= BC_NT) band_coef<1, false>(arrs, W, ldw, M, bm, C, xb, nx, nz, inv2, band_smem);
+  else band_coef<BC_NC, false>(arrs, W, ldw, M, bm, C, xb, nx, nz, inv2, band_smem);
+}
+
+// Blocks of 64 columns, each chunk's rows read while the one before is summed.
+__global__ void __launch_bounds__(BC_NT)
+    band_coef_ahead_kernel(const __grid_constant__ ArrayList arrs, const double* __restrict__ W, int ldw, int M, int bm,
+                           double* __restrict__ C, int nx, int nz, double inv2) {
+  extern __shared__ __align__(16) double2 band_smem[];
+  band_coef<1, true>(arrs, W, ldw, M, bm, C, blockIdx.y * BC_NT, nx, nz, inv2, band_smem);
 }
 
 // v[z][x] -= sum over the band's modes in order of (A_m cos_m(z) + B_m sin_m(z)),
@@ -535,25 +558,45 @@ __global__ void __launch_bounds__(BA_NT)
   else band_apply<2>(arrs, W, ldw, M, C, nx, nz, tw);
 }
 
-size_t band_coef_smem(int bm) { return sizeof(double2) * (size_t)bm * (2 * BD_CH + BD_TX); }
+size_t band_coef_smem(int bm, int cols) { return sizeof(double2) * (size_t)bm * (2 * BD_CH + cols); }
 
 cudaError_t launch_band(const ArrayList& arrs, int narr, const double* W, int ldw, int J, double* C, int nx, int nz,
                         double inv2, cudaStream_t s) {
-  const int M = J / 2, nxb = (nx + BD_TX - 1) / BD_TX;
-  // Modes per coefficient CTA.  Four CTAs fit an SM and all take equally long,
-  // so while they fill the SMs only a few times, the number whose turns come to
-  // the fewest modes (us at 256 x 512, modes 86..128: 105 against 112 with
-  // halving to four; 512 x 512 320 against 347); beyond, the most that fit,
-  // which read the array least (1024 x 2048 3.66 ms against 3.91).
+  const int M = J / 2, nxb = (nx + BD_TX - 1) / BD_TX, nxc = (nx + BC_NT - 1) / BC_NT;
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const long long slots = sms * 4;
-  auto turns = [&](int m) { return ((long long)((M + m - 1) / m) * nxb * narr + slots - 1) / slots; };
+  // Modes per CTA of the two-column form.  Four CTAs fit an SM and all take
+  // equally long, so while they fill the SMs only a few times, the number whose
+  // turns come to the fewest modes (us at 256 x 512, modes 86..128: 105 against
+  // 112 with halving to four; 512 x 512 320 against 347); beyond, the most that
+  // fit, which read the array least (1024 x 2048 3.66 ms against 3.91).
+  auto ctas = [&](int m, int blocks) { return (long long)((M + m - 1) / m) * blocks * narr; };
+  auto turns = [&](int m) { return (ctas(m, nxb) + slots - 1) / slots; };
   int bm = std::min(BC_BM, M);
   if (turns(bm) <= 4)
     for (int m = bm - 1; m >= 4; --m)
       if (turns(m) * m < turns(bm) * bm) bm = m;
-  band_coef_kernel<<<dim3((M + bm - 1) / bm, nxb, narr), BC_NT, band_coef_smem(bm), s>>>(arrs, W, ldw, M, bm, C, nx, nz, inv2);
+  // Few modes on a grid of few columns leave that form waiting for each chunk's
+  // rows: there the one-column form that reads a chunk ahead, with the fewest
+  // modes a CTA that keep four CTAs an SM (more of them read the array more often
+  // than they save).  It is taken when the busiest SM then has less to do: its
+  // column and mode costs 1.15 times as much, but the two-column form waits for
+  // its rows about as long as it sums 150 (filter us, two- against one-column
+  // form: 1024 x 128 13 modes 91 / 66, 8192 x 128 24 modes 813 / 585, 8192 x 448
+  // 13 modes 1328 / 1005, 8192 x 192 32 modes 1230 / 948, 1024 x 192 40 modes
+  // 183 / 158, but 1024 x 256 24 modes 129 / 137, 1024 x 768 13 modes 207 / 213,
+  // 1024 x 512 64 modes 462 / 512, one mode 4096 x 40 136 / 150).
+  int ba = 1;
+  while (ba < bm && ctas(ba, nxc) > slots) ++ba;
+  auto busiest = [&](int m, int blocks, int cols) { return (ctas(m, blocks) + sms - 1) / sms * m * cols; };
+  const long long two = busiest(bm, nxb, nx <= BC_NT ? BC_NT : BD_TX), one = busiest(ba, nxc, BC_NT);
+  if (ctas(ba, nxc) <= slots && one * 23 < (two + (nx > BC_NT ? 150 : 0)) * 20)
+    band_coef_ahead_kernel<<<dim3((M + ba - 1) / ba, nxc, narr), BC_NT, band_coef_smem(ba, BC_NT), s>>>(arrs, W, ldw, M, ba,
+                                                                                                     C, nx, nz, inv2);
+  else
+    band_coef_kernel<<<dim3((M + bm - 1) / bm, nxb, narr), BC_NT, band_coef_smem(bm, BD_TX), s>>>(arrs, W, ldw, M, bm, C, nx,
+                                                                                               nz, inv2);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   band_apply_kernel<<<dim3((nz + BD_CH - 1) / BD_CH, nxb, narr), BA_NT, 0, s>>>(arrs, W, ldw, M, C, nx, nz);
