@@ -523,39 +523,57 @@ bool col_fused_ok(const ymkh_ctx* c) {
   return column_fused_smem(c->nz, band_modes(c), p.suppress_kz0) <= kColumnFusedSmemMax;
 }
 
+int col_stages(const ymkh_ctx* c) {
+  const ymkh_params& p = c->prm;
+  return (p.xi_sponge > 0.0 || p.xi_cut > 0.0) + (p.suppress_kz0 != 0) + (c->nb > 0) + (p.hyp_diff_coeff > 0.0);
+}
+int col_modes(const ymkh_ctx* c) {
+  int m = 0;
+  for (int b = 0; b < c->nb; ++b) m += c->J[b] / 2;
+  return m;
+}
+
 // Whether a lone run takes that kernel: with two stages or more, or with band
 // filters alone up to 128 rows.  Step us, one kernel against separate ones:
-// all stages 64 x 768 54 / 72, 256 x 768 120 / 149, 512 x 1024 248 / 306;
-// z-mean and band 512 x 1024 664 / 686; band alone 64 x 192 35 / 43,
-// 96 x 512 56 / 59, but 256 x 512 169 / 161, 512 x 512 483 / 423 (its CTAs
-// have a column tile each and end unevenly); z-mean alone 256 x 256 55 / 54,
-// 512 x 1024 140 / 132.
+// all stages and 14 modes 64 x 768 53 / 63, 256 x 768 106 / 127, 512 x 1024 241
+// / 263; bands alone 64 x 192 36 / 37, 128 x 512 57 / 63, but 256 x 512 of 43
+// modes 158 / 136, 512 x 512 of 86 471 / 375 (its CTAs have a column tile each
+// and end unevenly); z-mean alone 256 x 256 43 / 41, 512 x 1024 134 / 127.
+// Above 48 modes and 256 rows a CTA lasts so long that what counts is how well
+// its turns fill the SMs: it is taken where they nearly do (z-mean and 86 modes
+// at 512 rows: 192 columns, 108 CTAs 182 / 187, 256 columns, 144 CTAs 192 / 203;
+// but 40 columns, 36 CTAs 178 / 102; hyperdiffusion and 86 modes 256 columns,
+// 168 CTAs 321 / 229, 1024 columns, 672 CTAs 782 / 706).
+constexpr int kColWideModes = 48;
 bool col_fused_alone(const ymkh_ctx* c) {
-  const ymkh_params& p = c->prm;
-  const int stages = (p.xi_sponge > 0.0 || p.xi_cut > 0.0) + (p.suppress_kz0 != 0) + (c->nb > 0) + (p.hyp_diff_coeff > 0.0);
+  const int stages = col_stages(c);
+  if (c->nz > 256 && col_modes(c) > kColWideModes) {
+    const int tiles = (c->nx + 31) / 32 * (c->prm.suppress_kz0 ? 18 : 21), turns = (tiles + c->sms - 1) / c->sms;
+    return stages >= 2 && tiles * 20 >= turns * c->sms * (turns == 1 ? 14 : 19);
+  }
   return stages >= 2 || (c->nb && c->nz <= 128);
 }
 
 // Whether a member of a batch does, where the launch is shared by all members of
-// its NZ: with 64 rows or less, two stages or more, or bands of up to 24 modes
-// in all; wider bands from 129 rows up only beside other stages and up to 256
-// rows.  Past 24 modes the separate band kernels, which run without a column
-// tile's uneven end, are ahead (step us, one kernel against separate ones, 4
-// and 12 runs: 256 x 512 bands of 16 modes 265 / 294, 724 / 830, 24 modes 323 /
-// 344, 881 / 965, 64 modes 611 / 565, 1686 / 1602; 512 x 512 16 modes 530 / 559,
-// 1489 / 1605, 24 modes 645 / 640, 1805 / 1851, 64 modes 1217 / 1069, 3413 /
-// 3117; z-mean and 86 modes 512 x 512 1316 / 1203, but 43 modes 256 x 512 417 /
-// 430; z-mean alone 64 x 768 69 / 77, 128 x 1024 135 / 129, 512 x 512 280 / 261;
-// z-mean and hyperdiffusion 512 x 512 279 / 297).
-constexpr int kColBatchModes = 24;
+// its NZ and its turns fill better: always with three stages or more, with two
+// but for more than 48 modes on large grids, with bands alone up to a number of
+// modes that falls with the columns, and with another stage alone on small
+// grids.  Step us of 4 and 12 runs, one kernel against separate ones: 512 x 512
+// z-mean and hyperdiffusion 280 / 299, 793 / 856, all stages with 40 modes 780 /
+// 776, 2273 / 2294; z-mean with 86 modes 512 x 512 1317 / 1188, 3888 / 3486, 512 x
+// 40 216 / 248, 583 / 666, with 40 modes 512 x 128 255 / 281, 713 / 779; bands
+// alone 512 x 512 14 modes 508 / 446, 1427 / 1283, 256 x 512 20 modes 300 / 282,
+// 815 / 788, 512 x 256 28 modes 394 / 355, 1081 / 991, 256 x 128 28 modes 145 /
+// 150, 332 / 381, 64 modes 224 / 196, 511 / 513; z-mean alone 64 x 512 58 / 63,
+// 132 / 153, 512 x 512 273 / 260, 777 / 743, sponge alone 128 x 40 50 / 52, 76 /
+// 85, 512 x 512 257 / 238, 731 / 681.
 bool col_fused_batch(const ymkh_ctx* c) {
   if (!c->col_ok) return false;
-  const ymkh_params& p = c->prm;
-  const int stages = (p.xi_sponge > 0.0 || p.xi_cut > 0.0) + (p.suppress_kz0 != 0) + (c->nb > 0) + (p.hyp_diff_coeff > 0.0);
-  int modes = 0;
-  for (int b = 0; b < c->nb; ++b) modes += c->J[b] / 2;
-  if (modes > kColBatchModes && c->nz > 128) return stages >= 2 && c->nz <= 256;
-  return modes > 0 || stages >= 2 || c->nz <= 64;
+  const int stages = col_stages(c), modes = col_modes(c);
+  if (stages >= 3) return true;
+  if (stages == 2) return c->nz <= 256 || c->nx < 128 || modes <= kColWideModes;
+  if (!modes) return c->nz <= 64 || c->nx < 512;
+  return c->nz <= 128 || modes <= (c->nx >= 512 ? 10 : c->nx >= 256 ? 24 : kColWideModes);
 }
 
 // How the fused FCT's items (strip-major segments) are cut into one contiguous
