@@ -163,7 +163,11 @@ int ymkh_set_fct_mode(ymkh_ctx* ctx, int mode);  /* YMKH_FCT_* (default FUSED); 
 /* Device time per stage over nsteps uncaptured steps (CUDA events between
  * stages on `stream`), accumulated in out_ms[0..6]: FCT, Maxwell,
  * sponge/xi_cut, z-mean, band filters, hyperdiffusion, colour-1 zeroing.
- * nout must be >= 7.  No reference counterpart. */
+ * Stages that share a kernel share a slot: where the column stages run as one
+ * kernel (NZ a multiple of 32 up to 512), all of it is in the band filters' slot,
+ * bands or not; the colour-1 zeroing is always in the z-mean's; and with the
+ * TF32 engine and suppress_kz0 the z-means are formed in the z-mean's slot and
+ * taken off in the band filters'.  nout must be >= 7.  No reference counterpart. */
 int ymkh_stage_times(ymkh_ctx* ctx, int nsteps, void* stream, float* out_ms, int nout);
 
 /* kernel_ym_init (ymgpu2d/YM_Init.cu:32-257) on the bound state; the
@@ -246,10 +250,12 @@ int ymkh_twiddles(int nz, int m_lo, int m_hi, float* cos_out, float* sin_out);
  * per process, ymgpu2d/scripts/*.sh).  Bound runs of any grid sizes and
  * parameters advance together: each step launches one FCT and one Maxwell
  * kernel over the (run, strip, segment) items of all members, then the
- * per-run filter stages.  A run's state after k batch steps is bit-identical
- * to k ymkh_step calls on it alone.  Membership may change between calls
- * (continuous batching); a run belongs to at most one batch at a time and
- * must not be stepped alone while it is a member. */
+ * column stages, in one launch per NZ for the members that share the kernel of
+ * them all.  A run's state after k batch steps is bit-identical to k ymkh_step
+ * calls on it alone.  Membership may change between calls (continuous
+ * batching); a run belongs to at most one batch at a time.  A member that was
+ * given a new state or new parameters, or was stepped alone, goes on from there
+ * (the caller orders the streams). */
 typedef struct ymkh_batch ymkh_batch;
 int ymkh_batch_create(ymkh_batch** out);
 int ymkh_batch_add(ymkh_batch* batch, ymkh_ctx* run);

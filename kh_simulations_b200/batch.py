@@ -1,11 +1,14 @@
 """``KHBatch``: many runs of any grid size advancing together.
 
 Each batch step launches one fused FCT kernel and one fused Maxwell kernel
-over the flattened (run, strip, segment) work list of every member, then
-the per-run filter stages (include/ymkh.h, ymkh_batch_*).  A run's state
-after k batch steps is bit-identical to k steps of the run alone.
-Membership may change between calls: that is what the serving loop uses
-for continuous batching.
+over the flattened (run, strip, segment) work list of every member, then the
+column stages (filters, z-mean, sponge, hyperdiffusion): one launch per NZ for
+the members that share the column kernel, the others' own kernels beside it on
+auxiliary streams (include/ymkh.h, ymkh_batch_*).  A run's state after k batch
+steps is bit-identical to k steps of the run alone.  Membership may change
+between calls, which is what the serving loop uses for continuous batching, and
+so may a member: given a new state or new parameters, or stepped alone, it goes
+on from there.
 """
 from __future__ import annotations
 

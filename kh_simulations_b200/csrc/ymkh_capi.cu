@@ -1210,8 +1210,10 @@ int ymkh_twiddles(int nz, int m_lo, int m_hi, float* cos_out, float* sin_out) tr
 
 // ------------------------------------------------------------------ batches
 // Runs of any sizes advance together: one FCT and one Maxwell launch per step
-// cover the (run, strip, segment) items of every member; the post-Maxwell
-// stages are launched per member.  Steps can be captured as CUDA graphs.
+// cover the (run, strip, segment) items of every member; one launch per NZ the
+// column stages of the members that share column_kernel (col_fused_batch), and
+// the others' stages are launched per member on auxiliary streams.  Steps can be
+// captured as CUDA graphs.
 
 struct ymkh_batch {
   std::vector<ymkh_ctx*> runs;
