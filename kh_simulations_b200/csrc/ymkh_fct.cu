@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(4 * TB, 2)
     else rows(HalfC<1>{});
     if (!bulk) {  // the next piece may take the stages by TMA
       cp_async_wait<0>();
-      fence_proxy_async();
+      if (T.nruns > 1) fence_proxy_async();  // (a run keeps to one kind of copy)
     }
   }
 }
@@ -1054,7 +1054,7 @@ __global__ void __launch_bounds__(F2_NT, 1) fct_strip_kernel(const __grid_consta
       }
       if (!bulk) {  // the next piece may take the slots by TMA
         cp_async_wait<0>();
-        fence_proxy_async();
+        if (T.nruns > 1) fence_proxy_async();  // (a run keeps to one kind of copy)
       }
       seq += (unsigned)nrow;
     }

@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(MX_NT, YMKH_MX_MINB)
     }
     if (!bulk) {  // the next item may take the stages by TMA
       cp_async_wait<0>();
-      fence_proxy_async();
+      if (T.nruns > 1) fence_proxy_async();  // (a run keeps to one kind of copy)
     }
   }
 }

@@ -27,10 +27,10 @@ def test_copied_piece_is_fenced_before_tma_may_take_its_slots(name, pieces):
     """A piece of rows copied with cp.async can be followed by one copied by
     TMA into the same slots (a batch of wall and periodic runs): every thread
     that copied ends the piece with its copies done and the fence."""
-    ends = re.findall(r"if \(!bulk\) \{? ?cp_async_wait<0>\(\);(.{0,24})", _code(name))
+    ends = re.findall(r"if \(!bulk\) \{? ?cp_async_wait<0>\(\);(.{0,44})", _code(name))
     assert len(ends) == pieces
     for after in ends:
-        assert after.startswith(" fence_proxy_async(); }"), after
+        assert after.startswith(" if (T.nruns > 1) fence_proxy_async(); }"), after  # a run keeps to one kind of copy
 
 
 def test_patched_columns_are_fenced_before_tma_retakes_the_slot():
