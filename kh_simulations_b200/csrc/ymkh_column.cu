@@ -332,11 +332,11 @@ cudaError_t prepare_column(int nz) {
 // the twiddles, which all lanes share, as one 16-byte (cos, sin) load.  That
 // load takes two shared-memory cycles: with one column a thread it could only
 // feed four FP64 instructions and set the pace (81% of the load pipe, FP64
-// 70%); with two, eight.  Measured there: 1.88 + 1.72 ms at 78% of the FP64
-// pipe each, against 4.58 ms for the two kernels that loaded both operands of
-// a 2 x 4 and a 4 x 4 block from shared memory; 512 x 1024 0.53 against 0.65
-// ms.  Staging the coefficients in shared memory too cost the apply kernel a
-// CTA per SM (2.28 ms).
+// 70%); with two, eight.  Measured there, with 21 arrays and under the profiler:
+// 2.18 + 2.11 ms at 78% of the FP64 pipe each, against 2.70 + 2.68 ms for the two
+// kernels that loaded both operands of a 2 x 4 and a 4 x 4 block from shared
+// memory.  Staging the coefficients in shared memory too cost the apply kernel a
+// CTA per SM.
 //
 // The reference's warp reduction (shfl_down by 16, 8, 4, 2, 1) leaves lane 0
 // with root = T4(0) + T4(1), T4(i) = T3(i) + T3(i+2), T3(i) = T2(i) + T2(i+4),
@@ -568,9 +568,10 @@ cudaError_t launch_band(const ArrayList& arrs, int narr, const double* W, int ld
   const long long slots = sms * 4;
   // Modes per CTA of the two-column form.  Four CTAs fit an SM and all take
   // equally long, so while they fill the SMs only a few times, the number whose
-  // turns come to the fewest modes (us at 256 x 512, modes 86..128: 105 against
-  // 112 with halving to four; 512 x 512 320 against 347); beyond, the most that
-  // fit, which read the array least (1024 x 2048 3.66 ms against 3.91).
+  // turns come to the fewest modes (us at 256 x 512, modes 86..128: 99 against 107
+  // with four and 105 with sixteen; 512 x 512, modes 171..256 314 against 347 and
+  // 342); beyond, the most that fit, which read the array least (1024 x 2048 3.65
+  // ms against 3.91 with four).
   auto ctas = [&](int m, int blocks) { return (long long)((M + m - 1) / m) * blocks * narr; };
   auto turns = [&](int m) { return (ctas(m, nxb) + slots - 1) / slots; };
   int bm = std::min(BC_BM, M);
